@@ -8,6 +8,7 @@ barriers pair CTAs by index).
 """
 from __future__ import annotations
 
+import itertools
 import os
 from dataclasses import dataclass, fields
 
@@ -19,6 +20,9 @@ def _env(name, default, cast):
     if cast is bool:
         return v not in ("0", "false", "False", "no")
     return cast(v)
+
+
+_versions = itertools.count(1)  # one number per change of any configuration object
 
 
 @dataclass
@@ -58,6 +62,11 @@ class Config:
     plan_cache_size: int = 512            # bound launches kept per communicator (least recently used go first)
     debug: bool = False
     debug_shrink_extent: int = 0          # test hook of the TCCL_DEBUG_CHECKS build: claim this many bytes less input
+
+    def __setattr__(self, name, value):
+        # bound launches are cached per `version`: any change of a field makes new plans
+        object.__setattr__(self, name, value)
+        object.__setattr__(self, "version", next(_versions))
 
     @classmethod
     def from_env(cls) -> "Config":

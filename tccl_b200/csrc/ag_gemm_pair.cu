@@ -343,8 +343,8 @@ ag_gemm_pair_kernel(const __grid_constant__ tccl_comm comm, const __grid_constan
   ag_gemm_pair_body(comm, p, blockIdx.x, gridDim.x);
 }
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
-ag_gemm_pair_kernel_emu(const tccl_comm* comms, const AgGemmPairParams* ps) {
-  ag_gemm_pair_body(comms[blockIdx.y], ps[blockIdx.y], blockIdx.x, gridDim.x);
+ag_gemm_pair_kernel_emu(const __grid_constant__ EmuParams<AgGemmPairParams> e) {
+  ag_gemm_pair_body(e.comm[blockIdx.y], e.args[blockIdx.y], blockIdx.x, gridDim.x);
 }
 
 static int fill_params(AgGemmPairParams* p, const tccl_ag_gemm_args* g, int world, int rank, uint64_t half_bytes) {
@@ -396,14 +396,13 @@ static int fill_params(AgGemmPairParams* p, const tccl_ag_gemm_args* g, int worl
 using namespace tccl::gemm;
 using namespace tccl::gemm2;
 
-extern "C" uint64_t tccl_ag_gemm_pair_param_bytes(void) { return sizeof(AgGemmPairParams); }
 
 // Same calling convention as tccl_allgather_gemm, except that every CTA moves data first: comm_ctas of
 // the arguments is the number of batches the shard goes out in (0 = 2); lsu_movers is a set of bits:
 // 2 = the diagnostic "move only", 4 = ring-ordered movers (ring_movers above).  `half_bytes`: distance in bytes from a_full[q] to the second
 // half of every rank's gathered buffer, or 0 when there is only one buffer (then the kernel opens
 // with a barrier).  l->grid must be even.
-extern "C" int tccl_allgather_gemm_pair(const tccl_comm* comm, const tccl_ag_gemm_args* args, void* dev_params,
+extern "C" int tccl_allgather_gemm_pair(const tccl_comm* comm, const tccl_ag_gemm_args* args,
                                         uint64_t half_bytes, const tccl_launch* l) {
   cudaStream_t s = reinterpret_cast<cudaStream_t>(l->stream);
   if (l->grid < 2 || (l->grid & 1)) return -TCCL_EINVAL;
@@ -423,15 +422,12 @@ extern "C" int tccl_allgather_gemm_pair(const tccl_comm* comm, const tccl_ag_gem
     return (int)cudaGetLastError();
   }
   const int W = l->n_emu;
-  if (W < 1 || W > TCCL_MAX_WORLD || !dev_params || ((uintptr_t)dev_params & 63)) return -TCCL_EINVAL;
-  AgGemmPairParams ps[TCCL_MAX_WORLD];
+  if (W < 1 || W > TCCL_MAX_WORLD) return -TCCL_EINVAL;
+  tccl::EmuParams<AgGemmPairParams> ep;
   for (int r = 0; r < W; ++r) {
-    int rc = fill_params(&ps[r], &args[r], W, r, half_bytes);
+    int rc = fill_params(&ep.args[r], &args[r], W, r, half_bytes);
     if (rc) return rc;
+    ep.comm[r] = comm[r];
   }
-  cudaError_t e = cudaMemcpyAsync(dev_params, ps, sizeof(AgGemmPairParams) * W, cudaMemcpyHostToDevice, s);
-  if (e != cudaSuccess) return (int)e;
-  const AgGemmPairParams* dps = reinterpret_cast<const AgGemmPairParams*>(dev_params);
-  return launch_pairs_emulated((const void*)ag_gemm_pair_kernel_emu, l->grid, W, kSmem2, s, (const void*)&comm,
-                               (const void*)&dps);
+  return launch_pairs_emulated((const void*)ag_gemm_pair_kernel_emu, l->grid, W, kSmem2, s, (const void*)&ep);
 }

@@ -174,8 +174,8 @@ extern "C" uint32_t tccl_allreduce_bulk_chunk_bytes(int world) { return bulk_chu
 
 // Inputs and destinations must be 16-byte aligned symmetric buffers; l->block must be 256.
 extern "C" int tccl_allreduce_twoshot_bulk(const tccl_comm* comm, const tccl_coll_args* args, const tccl_launch* l) {
-  const int world = l->n_emu ? l->n_emu : comm->world;
-  const int dtype = l->n_emu ? (l->meta & 0xff) : args->dtype;
+  const int world = comm->world;
+  const int dtype = args->dtype;
   if (l->block != kBulkThreads) return -TCCL_EINVAL;
   const size_t smem = (size_t)(kBulkInStages * world + kBulkOutStages) * bulk_chunk_bytes(world);
   if (l->n_emu == 0) {

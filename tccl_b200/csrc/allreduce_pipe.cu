@@ -190,12 +190,11 @@ static int launch_pipe_world(const tccl_comm* comm, const tccl_coll_args* args, 
 using namespace tccl;
 
 // The pipeline's shape (reducer warps, stages, unroll) sits in bits 8.. of args->flags for the
-// kernel and, identically, in bits 8.. of launch->meta for the host (in emulated mode `args`
-// is a device pointer the host cannot read).
+// kernel and, identically, in bits 8.. of launch->meta for the launcher.
 template <bool kNvls>
 static int pipe_entry(const tccl_comm* comm, const tccl_coll_args* args, const tccl_launch* l) {
-  const int world = l->n_emu ? l->n_emu : comm->world;
-  const int dtype = l->n_emu ? (l->meta & 0xff) : args->dtype;
+  const int world = comm->world;
+  const int dtype = args->dtype;
   const int pipe_flags = l->meta & ~0xff;
   if (l->n_emu == 0 && (args->flags & ~0xff) != pipe_flags) return -TCCL_EINVAL;
   switch (dtype) {

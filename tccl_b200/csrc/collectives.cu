@@ -550,20 +550,6 @@ template <typename T, int W> using ArPushNvls = AllReduceOneShotPush<T, W, true>
 
 using namespace tccl;
 
-// The launchers pick a template instance by world size and dtype.  In emulated
-// mode `comm`/`args` are device pointers the host cannot read, so the world size
-// is n_emu and the dtype comes in the launch struct's `meta` field.
-static inline void host_meta(const tccl_comm* comm, const tccl_coll_args* args, const tccl_launch* l, int* world,
-                             int* dtype) {
-  if (l->n_emu == 0) {
-    *world = comm->world;
-    *dtype = args ? args->dtype : 0;
-  } else {
-    *world = l->n_emu;
-    *dtype = l->meta & 0xff;
-  }
-}
-
 extern "C" {
 
 uint64_t tccl_push_slot_bytes(uint64_t ll_bytes, int world) {
@@ -585,9 +571,7 @@ int tccl_wait_never(const tccl_comm* comm, const tccl_barrier_args* args, const 
 
 #define TCCL_COLL(name, Op)                                                                   \
   int name(const tccl_comm* comm, const tccl_coll_args* args, const tccl_launch* l) {         \
-    int world, dtype;                                                                         \
-    host_meta(comm, args, l, &world, &dtype);                                                 \
-    return dispatch<Op>(comm, args, l, world, dtype);                                         \
+    return dispatch<Op>(comm, args, l, comm->world, args->dtype);                             \
   }
 TCCL_COLL(tccl_allreduce_oneshot_p2p, AllReduceOneShotP2P)
 TCCL_COLL(tccl_allreduce_oneshot_nvls, AllReduceOneShotNvls)

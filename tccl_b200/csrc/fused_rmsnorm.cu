@@ -179,10 +179,10 @@ static int launch_by_width(const tccl_comm* comm, const tccl_arn_args* args, con
   return -TCCL_ESIZE;
 }
 
-// `hidden` is passed separately because in emulated mode `args` is a device pointer.
 extern "C" int tccl_allreduce_bias_residual_rmsnorm(const tccl_comm* comm, const tccl_arn_args* args, int nvls,
-                                                    int hidden, const tccl_launch* l) {
-  const int dtype = l->n_emu ? (l->meta & 0xff) : args->dtype;
+                                                    const tccl_launch* l) {
+  const int hidden = args->hidden;
+  const int dtype = args->dtype;
   if (nvls) {
     switch (dtype) {
       case TCCL_BF16: return launch_by_width<__nv_bfloat16, true>(comm, args, l, hidden);

@@ -47,9 +47,8 @@ inline int make_tmap_bf16_kmajor(CUtensorMap* map, const void* base, int rows, i
 // resident together: a cooperative launch guarantees that or fails cleanly; where the runtime does
 // not take a cooperative launch of a cluster kernel, the launch goes ahead only if the occupancy
 // query says that every cluster fits at once.
-inline int launch_pairs_emulated(const void* fn, int grid, int world, size_t smem, cudaStream_t s, const void* arg0,
-                                 const void* arg1) {
-  void* kargs[2] = {const_cast<void*>(arg0), const_cast<void*>(arg1)};
+inline int launch_pairs_emulated(const void* fn, int grid, int world, size_t smem, cudaStream_t s, const void* params) {
+  void* kargs[1] = {const_cast<void*>(params)};
   cudaError_t e = cudaLaunchCooperativeKernel(fn, dim3(grid, world), dim3(256), kargs, smem, s);
   if (e == cudaSuccess) return 0;
   if (e != cudaErrorInvalidValue && e != cudaErrorNotSupported && e != cudaErrorInvalidConfiguration &&

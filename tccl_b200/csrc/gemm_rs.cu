@@ -207,8 +207,8 @@ __global__ void __launch_bounds__(kThreads, 1)
 gemm_rs_kernel(const __grid_constant__ tccl_comm comm, const __grid_constant__ GemmRsParams p) {
   gemm_rs_body(comm, p, blockIdx.x, gridDim.x);
 }
-__global__ void __launch_bounds__(kThreads, 1) gemm_rs_kernel_emu(const tccl_comm* comms, const GemmRsParams* ps) {
-  gemm_rs_body(comms[blockIdx.y], ps[blockIdx.y], blockIdx.x, gridDim.x);
+__global__ void __launch_bounds__(kThreads, 1) gemm_rs_kernel_emu(const __grid_constant__ EmuParams<GemmRsParams> e) {
+  gemm_rs_body(e.comm[blockIdx.y], e.args[blockIdx.y], blockIdx.x, gridDim.x);
 }
 
 static int fill_params(GemmRsParams* p, const tccl_gemm_rs_args* g, int world) {
@@ -238,13 +238,8 @@ using namespace tccl::gemm;
 extern "C" uint64_t tccl_gemm_rs_stage_bytes(int m, int n, int world) {
   return (uint64_t)world * (uint64_t)(m / world / BM) * (uint64_t)(n / BN) * kSlotBytes;
 }
-extern "C" uint64_t tccl_gemm_rs_param_bytes(void) { return sizeof(GemmRsParams); }
 
-// real mode: `comm` and `args` are host structs of the calling rank, `dev_params` unused.
-// emulated mode: `comm` is the device array of W communicators, `args` a HOST array of W
-// argument structs, `dev_params` device scratch of W * tccl_gemm_rs_param_bytes() bytes
-// (64-byte aligned) that receives the kernels' parameter blocks.
-extern "C" int tccl_gemm_reduce_scatter(const tccl_comm* comm, const tccl_gemm_rs_args* args, void* dev_params,
+extern "C" int tccl_gemm_reduce_scatter(const tccl_comm* comm, const tccl_gemm_rs_args* args,
                                         uint64_t stage_bytes, const tccl_launch* l) {
   cudaStream_t s = reinterpret_cast<cudaStream_t>(l->stream);
   if (l->grid <= 0) return -TCCL_EINVAL;
@@ -265,17 +260,15 @@ extern "C" int tccl_gemm_reduce_scatter(const tccl_comm* comm, const tccl_gemm_r
     return (int)cudaGetLastError();
   }
   const int W = l->n_emu;
-  if (W < 1 || W > TCCL_MAX_WORLD || !dev_params || ((uintptr_t)dev_params & 63)) return -TCCL_EINVAL;
+  if (W < 1 || W > TCCL_MAX_WORLD) return -TCCL_EINVAL;
   if (tccl_gemm_rs_stage_bytes(args[0].m, args[0].n, W) > stage_bytes) return -TCCL_ESIZE;
-  GemmRsParams ps[TCCL_MAX_WORLD];
+  tccl::EmuParams<GemmRsParams> ep;
   for (int r = 0; r < W; ++r) {
-    int rc = fill_params(&ps[r], &args[r], W);
+    int rc = fill_params(&ep.args[r], &args[r], W);
     if (rc) return rc;
+    ep.comm[r] = comm[r];
   }
-  cudaError_t e = cudaMemcpyAsync(dev_params, ps, sizeof(GemmRsParams) * W, cudaMemcpyHostToDevice, s);
-  if (e != cudaSuccess) return (int)e;
-  const GemmRsParams* dps = reinterpret_cast<const GemmRsParams*>(dev_params);
-  void* kargs[2] = {(void*)&comm, (void*)&dps};
+  void* kargs[1] = {(void*)&ep};
   return (int)cudaLaunchCooperativeKernel((const void*)gemm_rs_kernel_emu, dim3(l->grid, W), dim3(kThreads), kargs,
                                           kSmemBytes, s);
 }

@@ -277,8 +277,8 @@ gemm_rs_pair_kernel(const __grid_constant__ tccl_comm comm, const __grid_constan
   gemm_rs_pair_body(comm, p, blockIdx.x, gridDim.x);
 }
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
-gemm_rs_pair_kernel_emu(const tccl_comm* comms, const GemmRsPairParams* ps) {
-  gemm_rs_pair_body(comms[blockIdx.y], ps[blockIdx.y], blockIdx.x, gridDim.x);
+gemm_rs_pair_kernel_emu(const __grid_constant__ EmuParams<GemmRsPairParams> e) {
+  gemm_rs_pair_body(e.comm[blockIdx.y], e.args[blockIdx.y], blockIdx.x, gridDim.x);
 }
 
 static int fill_params(GemmRsPairParams* p, const tccl_gemm_rs_args* g, int world, uint64_t stage_bytes, int sync_entry) {
@@ -313,11 +313,10 @@ using namespace tccl::gemm2;
 extern "C" uint64_t tccl_gemm_rs_pair_stage_bytes(int m, int n, int world) {
   return 2ull * (uint64_t)world * (uint64_t)(m / world / 128) * (uint64_t)(n / BN2) * kSlotBytes2 + 2048;
 }
-extern "C" uint64_t tccl_gemm_rs_pair_param_bytes(void) { return sizeof(GemmRsPairParams); }
 
 // Same calling convention as tccl_gemm_reduce_scatter; l->meta bit 8 (TCCL_RS_SYNC_ENTRY) asks for
 // the entry barrier.  l->grid must be even.
-extern "C" int tccl_gemm_reduce_scatter_pair(const tccl_comm* comm, const tccl_gemm_rs_args* args, void* dev_params,
+extern "C" int tccl_gemm_reduce_scatter_pair(const tccl_comm* comm, const tccl_gemm_rs_args* args,
                                              uint64_t stage_bytes, const tccl_launch* l) {
   cudaStream_t s = reinterpret_cast<cudaStream_t>(l->stream);
   if (l->grid < 2 || (l->grid & 1)) return -TCCL_EINVAL;
@@ -338,15 +337,12 @@ extern "C" int tccl_gemm_reduce_scatter_pair(const tccl_comm* comm, const tccl_g
     return (int)cudaGetLastError();
   }
   const int W = l->n_emu;
-  if (W < 1 || W > TCCL_MAX_WORLD || !dev_params || ((uintptr_t)dev_params & 63)) return -TCCL_EINVAL;
-  GemmRsPairParams ps[TCCL_MAX_WORLD];
+  if (W < 1 || W > TCCL_MAX_WORLD) return -TCCL_EINVAL;
+  tccl::EmuParams<GemmRsPairParams> ep;
   for (int r = 0; r < W; ++r) {
-    int rc = fill_params(&ps[r], &args[r], W, stage_bytes, sync_entry);
+    int rc = fill_params(&ep.args[r], &args[r], W, stage_bytes, sync_entry);
     if (rc) return rc;
+    ep.comm[r] = comm[r];
   }
-  cudaError_t e = cudaMemcpyAsync(dev_params, ps, sizeof(GemmRsPairParams) * W, cudaMemcpyHostToDevice, s);
-  if (e != cudaSuccess) return (int)e;
-  const GemmRsPairParams* dps = reinterpret_cast<const GemmRsPairParams*>(dev_params);
-  return launch_pairs_emulated((const void*)gemm_rs_pair_kernel_emu, l->grid, W, kSmem2, s, (const void*)&comm,
-                               (const void*)&dps);
+  return launch_pairs_emulated((const void*)gemm_rs_pair_kernel_emu, l->grid, W, kSmem2, s, (const void*)&ep);
 }

@@ -104,7 +104,7 @@ struct QuantAllReduce {
     const char* in = reinterpret_cast<const char*>(a.in);
     char* out = reinterpret_cast<char*>(a.out);
 
-    barrier_p2p(c, bid, deadline);  // the staging area's previous user is done on every rank
+    barrier_any(c, bid, deadline, false);  // the staging area's previous user is done on every rank
 
     // ---- 1: quantise the own input, chunk by chunk, into the owners' slots [me]
     for (int k = 0; k < W; ++k) {
@@ -140,7 +140,7 @@ struct QuantAllReduce {
           st_relaxed_sys(reinterpret_cast<uint32_t*>(c.stage[q] + off_ps) + (uint64_t)me * cps + j, __float_as_uint(scale));
       }
     }
-    barrier_p2p(c, bid, deadline);  // all partials of this CTA's chunks have landed at their owners
+    barrier_any(c, bid, deadline, false);  // all partials of this CTA's chunks have landed at their owners
 
     // ---- 2: sum the W copies of the own chunks in fp32, quantise the sum, store it to every rank
     const char* mine = c.stage[me];
@@ -182,7 +182,7 @@ struct QuantAllReduce {
         if (lane == 0) st_relaxed_sys(reinterpret_cast<uint32_t*>(c.stage[p] + off_ss) + ch, __float_as_uint(scale));
       }
     }
-    barrier_p2p(c, bid, deadline);  // all sums of this CTA's chunks have landed everywhere
+    barrier_any(c, bid, deadline, false);  // all sums of this CTA's chunks have landed everywhere
 
     // ---- 3: dequantise every slice's chunks of this warp into the output
     for (int q = 0; q < W; ++q) {

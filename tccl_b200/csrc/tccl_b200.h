@@ -10,9 +10,10 @@
  *  - "real" mode (n_emu == 0): `comm` / `args` point to ONE struct in host
  *    memory describing the calling rank.
  *  - "emulated" mode (n_emu == W >= 1): `comm` / `args` point to arrays of W
- *    structs in DEVICE memory; one cooperative launch with gridDim.y == W runs
- *    all W ranks on the current GPU (blockIdx.y is the rank).  This is how the
- *    multi-rank protocols are exercised on a single GPU.
+ *    structs, in host memory too (they travel as the kernel's parameter); one
+ *    cooperative launch with gridDim.y == W runs all W ranks on the current GPU
+ *    (blockIdx.y is the rank).  This is how the multi-rank protocols are
+ *    exercised on a single GPU.
  *  - Device-side waits are bounded by `timeout_ns`; a wait that runs out
  *    records a status (see tccl_status_word) and the kernel returns.
  */
@@ -132,8 +133,7 @@ typedef struct tccl_launch {
   int32_t grid;    /* CTAs per rank */
   int32_t block;   /* threads per CTA */
   int32_t n_emu;   /* 0 = real, W = emulate W ranks on this GPU */
-  int32_t meta;    /* bits 0-7: tccl_dtype of the args (read in emulated mode, where they are device-resident);
-                      bits 8..: kernel-specific shape bits (TCCL_F_PIPE_*) */
+  int32_t meta;    /* bits 0-7: unused; bits 8..: kernel-specific shape bits (TCCL_F_PIPE_*) */
   void* stream;    /* cudaStream_t */
 } tccl_launch;
 
@@ -244,9 +244,7 @@ typedef struct tccl_arn_args {
   int32_t dtype;
   int32_t flags;                   /* TCCL_F_NVLS_BARRIER */
 } tccl_arn_args;
-/* `hidden` repeats args->hidden for the host (in emulated mode `args` is a device pointer) */
-int tccl_allreduce_bias_residual_rmsnorm(const tccl_comm*, const tccl_arn_args*, int nvls, int hidden,
-                                         const tccl_launch*);
+int tccl_allreduce_bias_residual_rmsnorm(const tccl_comm*, const tccl_arn_args*, int nvls, const tccl_launch*);
 
 /* ---- tcgen05 GEMM (bf16 in, fp32 accumulate in tensor memory, bf16 out) ---- */
 typedef struct tccl_gemm_args {
@@ -274,11 +272,7 @@ typedef struct tccl_gemm_rs_args {
 } tccl_gemm_rs_args;
 /* bytes of staging area (per rank) the fused kernel needs for an m x n product */
 uint64_t tccl_gemm_rs_stage_bytes(int m, int n, int world);
-uint64_t tccl_gemm_rs_param_bytes(void);
-/* real mode: comm/args are host structs, dev_params unused.  Emulated mode: comm is the
- * device array of communicators, args a HOST array of n_emu structs, dev_params device
- * scratch of n_emu * tccl_gemm_rs_param_bytes() bytes (64-byte aligned). */
-int tccl_gemm_reduce_scatter(const tccl_comm* comm, const tccl_gemm_rs_args* args, void* dev_params,
+int tccl_gemm_reduce_scatter(const tccl_comm* comm, const tccl_gemm_rs_args* args,
                              uint64_t stage_bytes, const tccl_launch* l);
 
 /* Same product on CTA pairs (tcgen05.mma.cta_group::2), tiles interleaved over the owners so that the
@@ -287,8 +281,7 @@ int tccl_gemm_reduce_scatter(const tccl_comm* comm, const tccl_gemm_rs_args* arg
  * barrier (needed when the previous user of the staging area was another kernel). */
 #define TCCL_RS_SYNC_ENTRY 256
 uint64_t tccl_gemm_rs_pair_stage_bytes(int m, int n, int world);
-uint64_t tccl_gemm_rs_pair_param_bytes(void);
-int tccl_gemm_reduce_scatter_pair(const tccl_comm* comm, const tccl_gemm_rs_args* args, void* dev_params,
+int tccl_gemm_reduce_scatter_pair(const tccl_comm* comm, const tccl_gemm_rs_args* args,
                                   uint64_t stage_bytes, const tccl_launch* l);
 
 /* ---- fused all-gather -> GEMM (rows gathered over the ranks) -------------- */
@@ -312,9 +305,8 @@ typedef struct tccl_ag_gemm_args {
                                        128).  NULL: own rows first, then the peers' rows in arrival order */
 } tccl_ag_gemm_args;
 #define TCCL_AG_UNIT(mt, nt, half) ((int32_t)(mt) | ((int32_t)(nt) << 12) | ((int32_t)(half) << 28))
-uint64_t tccl_ag_gemm_param_bytes(void);
 /* same calling convention as tccl_gemm_reduce_scatter */
-int tccl_allgather_gemm(const tccl_comm* comm, const tccl_ag_gemm_args* args, void* dev_params,
+int tccl_allgather_gemm(const tccl_comm* comm, const tccl_ag_gemm_args* args,
                         const tccl_launch* l);
 
 /* Same product on CTA pairs (tcgen05.mma.cta_group::2); every CTA moves its share of the shard first
@@ -322,8 +314,7 @@ int tccl_allgather_gemm(const tccl_comm* comm, const tccl_ag_gemm_args* args, vo
  * destination with plain stores instead of batch by batch to all ranks).  m % (world * 256) == 0; l->grid even.  `half_bytes`: distance
  * from a_full[q] to the second half of every rank's gathered buffer — the halves alternate from call to
  * call and no entry barrier is needed — or 0 for a single buffer (the kernel then opens with a barrier). */
-uint64_t tccl_ag_gemm_pair_param_bytes(void);
-int tccl_allgather_gemm_pair(const tccl_comm* comm, const tccl_ag_gemm_args* args, void* dev_params,
+int tccl_allgather_gemm_pair(const tccl_comm* comm, const tccl_ag_gemm_args* args,
                              uint64_t half_bytes, const tccl_launch* l);
 
 #ifdef __cplusplus

@@ -250,7 +250,7 @@ using namespace tccl;
 extern "C" int tccl_tree_max_ctas(uint64_t tree_bytes) { return tree_max_ctas(tree_bytes); }
 
 extern "C" int tccl_allreduce_tree(const tccl_comm* comm, const tccl_tree_args* args, const tccl_launch* l) {
-  const int dtype = l->n_emu ? (l->meta & 0xff) : args->dtype;
+  const int dtype = args->dtype;
   if (l->n_emu == 0) {
     const int K = args->ctas_per_role;
     if (K < 1 || K > tree_max_ctas(comm->tree_bytes) || l->grid != 4 * K) return -TCCL_ESIZE;

@@ -176,7 +176,7 @@ using namespace tccl;
 // TCCL_TREE_LL_MAX_CTAS.  args->buf[rank] (this rank's own result buffer, for the in-place form) and
 // args->out may each be null; the other entries of buf are not used.
 extern "C" int tccl_allreduce_tree_ll(const tccl_comm* comm, const tccl_tree_args* args, const tccl_launch* l) {
-  const int dtype = l->n_emu ? (l->meta & 0xff) : args->dtype;
+  const int dtype = args->dtype;
   if (l->n_emu == 0) {
     const int K = args->ctas_per_role;
     const uint64_t esz = args->dtype == TCCL_F32 ? 4 : 2;

@@ -15,6 +15,7 @@ import torch
 from ..parallel.world import WorldBase
 from ..utils import lib as L
 from ._common import K, check_sym_tensor, dtype_code, get_world
+from .collectives import _planned
 
 __all__ = ["gemm_reduce_scatter", "all_gather_gemm", "all_reduce_bias_residual_rmsnorm", "pack_gate_up",
            "ag_pair_schedule"]
@@ -23,9 +24,13 @@ __all__ = ["gemm_reduce_scatter", "all_gather_gemm", "all_reduce_bias_residual_r
 def _locals(w: WorldBase, x):
     """Per-rank local tensors of an ordinary (non symmetric) argument: a tensor in
     a real world, a list/EmuTensor of W tensors in an emulated one."""
-    if w.plans is not None:  # a real world drives exactly one rank
-        return {w.local_ranks[0]: x}
-    return {r: x[r] for r in w.local_ranks}
+    if w.emulated:
+        return [x[r] for r in w.local_ranks]
+    return [x]  # a real world drives exactly one rank
+
+
+def _tkeys(ts) -> tuple:
+    return tuple([(t.data_ptr(), t.shape, t.stride(), t.dtype) for t in ts])
 
 
 def _trace_ptr(w: WorldBase, trace, r: int, grid: int) -> int:
@@ -33,15 +38,46 @@ def _trace_ptr(w: WorldBase, trace, r: int, grid: int) -> int:
     emulated) that receives per-tile %globaltimer stamps; None = no tracing."""
     if trace is None:
         return 0
-    t = trace if w.plans is not None else trace[r]
+    t = trace[r] if w.emulated else trace
     if t.dtype != torch.int64 or t.numel() < grid * 64 or not t.is_cuda:
         raise ValueError(f"trace must be an int64 CUDA tensor of >= {grid * 64} words")
     return t.data_ptr()
 
 
+class FusedPlan:
+    """A bound launch of a fused kernel: validated argument structs, one per local rank in one array, and the
+    launcher.  Holds raw addresses, no tensors (see ``collectives.Plan``); ``fresh`` = (shape, strides) of the
+    output that a call allocates when the caller gives none."""
+
+    __slots__ = ("arr", "l", "call", "name", "fresh", "user", "views")
+
+    def __init__(self, w: WorldBase, name: str, arr, grid: int, block: int, extra=(), fresh=None, user=None):
+        self.arr, self.name, self.fresh, self.user, self.views = arr, name, fresh, user, None
+        self.l = l = L.Launch(grid, block, len(arr) if w.emulated else 0, 0, None)
+        fn, refs = getattr(L.lib(), name), (w.comm_ref(), C.byref(arr), *extra, C.byref(l))
+        self.call = lambda: fn(*refs)
+
+    def outputs(self, like):
+        """New outputs next to the tensors ``like``, written into the argument structs."""
+        shape, strides = self.fresh
+        outs = []
+        for g, t in zip(self.arr, like):
+            o = torch.empty_strided(shape, strides, dtype=torch.bfloat16, device=t.device)
+            g.out = o.data_ptr()
+            outs.append(o)
+        return outs
+
+    def go(self, w: WorldBase, device) -> None:
+        self.l.stream = torch._C._cuda_getCurrentRawStream(device.index)
+        rc = self.call()
+        if rc:
+            L.check(rc, self.name)
+        w.launches += 1
+
+
 def _gemm_ctas(w: WorldBase, pairs: bool = False) -> int:
     n = w.config.max_ctas or w.num_sms()
-    if w.plans is None:  # emulated ranks share one GPU and each CTA takes a whole SM
+    if w.emulated:  # the ranks share one GPU and each CTA takes a whole SM
         n = max(1, w.num_sms() // w.world_size)
     return max(2, n & ~1) if pairs else n
 
@@ -68,9 +104,25 @@ def gemm_reduce_scatter(a, bt, out=None, *, trace=None, variant: str = "auto", w
     mainloop, no entry barrier (needs ``M % (256 W) == 0`` and twice the staging space);
     ``"single"`` = 128 x 256 single-CTA tiles; ``"auto"`` = pair when the shape allows."""
     w = get_world(world)
-    W = w.world_size
     As, Bs = _locals(w, a), _locals(w, bt)
-    a0, b0 = As[w.local_ranks[0]], Bs[w.local_ranks[0]]
+    Os = _locals(w, out) if out is not None else None
+    key = ("gemm_rs", _tkeys(As), _tkeys(Bs), Os and _tkeys(Os), variant)
+    p = _planned(w, key, _plan_gemm_rs, As, Bs, Os, variant)
+    grid = p.l.grid
+    for i, r in enumerate(w.local_ranks):
+        p.arr[i].trace = _trace_ptr(w, trace, r, grid) if trace is not None else 0
+    handoff = _stage_handoff(w, p.user)
+    p.l.meta = K["TCCL_RS_SYNC_ENTRY"] if handoff and p.user == "gemm_rs_pair" else 0
+    outs = Os if Os is not None else p.outputs(As)
+    p.go(w, As[0].device)
+    if out is not None:
+        return out
+    return outs if w.emulated else outs[0]
+
+
+def _plan_gemm_rs(w, As, Bs, Os, variant) -> FusedPlan:
+    W = w.world_size
+    a0, b0 = As[0], Bs[0]
     if a0.dtype != torch.bfloat16 or b0.dtype != torch.bfloat16:
         raise TypeError("gemm_reduce_scatter takes bfloat16 operands")
     M, Kr = a0.shape
@@ -80,8 +132,7 @@ def gemm_reduce_scatter(a, bt, out=None, *, trace=None, variant: str = "auto", w
     if M % (W * 128) or N % 256 or Kr % 8:
         raise ValueError(f"need M % {W * 128} == 0, N % 256 == 0, K % 8 == 0 (got M={M}, N={N}, K={Kr})")
     lib = L.lib()
-    for f in ("tccl_gemm_rs_stage_bytes", "tccl_gemm_rs_param_bytes", "tccl_gemm_rs_pair_stage_bytes",
-              "tccl_gemm_rs_pair_param_bytes"):
+    for f in ("tccl_gemm_rs_stage_bytes", "tccl_gemm_rs_pair_stage_bytes"):
         getattr(lib, f).restype = C.c_uint64
     stage_bytes = (w.config.stage_mb << 20) - w.ll_bytes
     if variant not in ("auto", "pair", "single"):
@@ -95,40 +146,15 @@ def gemm_reduce_scatter(a, bt, out=None, *, trace=None, variant: str = "auto", w
     if need > stage_bytes:
         raise ValueError(f"staging area too small: need {need >> 20} MiB, have {w.config.stage_mb} MiB "
                          "(raise TCCL_STAGE_MB)")
-    outs = {}
-    grid = _gemm_ctas(w, pair)
-    meta = 0
-    if pair:
-        meta = K["TCCL_RS_SYNC_ENTRY"] if _stage_handoff(w, "gemm_rs_pair") else 0
-    else:
-        _stage_handoff(w, "gemm_rs")
-    Os = _locals(w, out) if out is not None else None
-    arr = (L.GemmRsArgs * len(w.local_ranks))()
-    for i, r in enumerate(w.local_ranks):
-        ar, br = As[r], Bs[r]
+    arr = (L.GemmRsArgs * len(As))()
+    for i, (ar, br) in enumerate(zip(As, Bs)):
         if ar.stride(1) != 1 or br.stride(1) != 1:
             raise ValueError("operands must have a unit inner stride")
-        o = Os[r] if Os is not None else torch.empty((M // W, N), dtype=torch.bfloat16, device=ar.device)
-        outs[r] = o
-        arr[i] = L.GemmRsArgs(ar.data_ptr(), br.data_ptr(), o.data_ptr(), M, N, Kr, ar.stride(0), br.stride(0),
-                              o.stride(0), _trace_ptr(w, trace, r, grid))
-    stream = torch.cuda.current_stream(a0.device).cuda_stream
-    fn = lib.tccl_gemm_reduce_scatter_pair if pair else lib.tccl_gemm_reduce_scatter
-    if w.plans is not None:
-        l = L.Launch(grid, 256, 0, meta, C.c_void_p(stream))
-        rc = fn(C.byref(w.comm), C.byref(arr[0]), None, C.c_uint64(stage_bytes), C.byref(l))
-    else:
-        pb = int(lib.tccl_gemm_rs_pair_param_bytes() if pair else lib.tccl_gemm_rs_param_bytes())
-        scratch = torch.empty(pb * W + 64, dtype=torch.uint8, device=a0.device)
-        base = (scratch.data_ptr() + 63) & ~63
-        w._keep.append(scratch)
-        l = L.Launch(grid, 256, W, meta, C.c_void_p(stream))
-        rc = fn(C.c_void_p(w.comms_dev.data_ptr()), arr, C.c_void_p(base), C.c_uint64(stage_bytes), C.byref(l))
-    L.check(rc, "tccl_gemm_reduce_scatter_pair" if pair else "tccl_gemm_reduce_scatter")
-    w.launches += 1
-    if out is not None:
-        return out
-    return [outs[r] for r in w.local_ranks] if w.plans is None else outs[w.local_ranks[0]]
+        optr, ldo = (Os[i].data_ptr(), Os[i].stride(0)) if Os is not None else (0, N)
+        arr[i] = L.GemmRsArgs(ar.data_ptr(), br.data_ptr(), optr, M, N, Kr, ar.stride(0), br.stride(0), ldo, 0)
+    name = "tccl_gemm_reduce_scatter_pair" if pair else "tccl_gemm_reduce_scatter"
+    return FusedPlan(w, name, arr, _gemm_ctas(w, pair), 256, (C.c_uint64(stage_bytes),), ((M // W, N), (N, 1)),
+                     "gemm_rs_pair" if pair else "gemm_rs")
 
 
 def ag_pair_schedule(W: int, rank: int, tm: int, tn: int, pairs: int, nbatch: int, k: int, *, halves: bool = True,
@@ -226,9 +252,27 @@ def all_gather_gemm(a_shard, bt, a_full=None, out=None, *, comm_ctas: int = 0, s
     needs no barrier on entry): the returned ``a_full`` is the one this call filled, and it stays
     valid until the call after the next one."""
     w = get_world(world)
-    W = w.world_size
     As, Bs = _locals(w, a_shard), _locals(w, bt)
-    a0, b0 = As[w.local_ranks[0]], Bs[w.local_ranks[0]]
+    Os = _locals(w, out) if out is not None else None
+    opts = (comm_ctas, swiglu, int(lsu_movers), variant)
+    key = ("ag_gemm", _tkeys(As), _tkeys(Bs), Os and _tkeys(Os), None if a_full is None else w.tkey(a_full), opts)
+    p = _planned(w, key, _plan_ag_gemm, As, Bs, a_full, Os, *opts)
+    grid = p.l.grid
+    for i, r in enumerate(w.local_ranks):
+        p.arr[i].trace = _trace_ptr(w, trace, r, grid) if trace is not None else 0
+    outs = Os if Os is not None else p.outputs(As)
+    p.go(w, As[0].device)
+    seq = 0
+    if p.user == "ag_gemm_pair":  # mirrors the device's count of pair calls, which picks the half (see reset())
+        seq = w.__dict__.get("_ag_seq", 0)
+        w.__dict__["_ag_seq"] = seq + 1
+    res = out if out is not None else (outs if w.emulated else outs[0])
+    return res, (a_full if a_full is not None else p.views[seq % len(p.views)])
+
+
+def _plan_ag_gemm(w, As, Bs, a_full, Os, comm_ctas, swiglu, lsu_movers, variant) -> FusedPlan:
+    W = w.world_size
+    a0, b0 = As[0], Bs[0]
     if a0.dtype != torch.bfloat16 or b0.dtype != torch.bfloat16:
         raise TypeError("all_gather_gemm takes bfloat16 operands")
     rows, Kd = a0.shape
@@ -247,31 +291,19 @@ def all_gather_gemm(a_shard, bt, a_full=None, out=None, *, comm_ctas: int = 0, s
         raise ValueError("the pair kernel needs (M / W) % 256 == 0")
     pair = pair_ok and variant != "single"
     half_bytes = 0
-    ret_full = a_full
-    seq = 0
-    if pair:  # mirrors the device's count of pair calls, which picks the half (see reset())
-        seq = w.__dict__.get("_ag_seq", 0)
-        w.__dict__["_ag_seq"] = seq + 1
+    views = None
     if a_full is None:
         cache = w.__dict__.setdefault("_ag_buffers", {})
         key = (M, Kd, pair)
         a_full = cache.get(key)
         if a_full is None:
             a_full = cache[key] = w.empty((2, M, Kd) if pair else (M, Kd), torch.bfloat16)
-        ret_full = a_full
-        if pair:
-            half_bytes = M * Kd * 2
-            if w.plans is not None:
-                ret_full = a_full[seq & 1]
-            else:
-                from ..parallel.emu import EmuTensor
-                ret_full = EmuTensor([t[seq & 1] for t in a_full.parts])
+        half = a_full.half if w.emulated else a_full.__getitem__
+        views = [half(0), half(1)] if pair else [a_full]
+        half_bytes = M * Kd * 2 if pair else 0
     full_ptrs = w.peer_ptrs(a_full)
     # two ranks: the switch would deliver every row to its sender too (twice the inbound bytes of a plain store)
     mc = w.mc_ptr(a_full) if ((W > 2 and not w.config.ag_ring) or not pair) else 0
-    lib = L.lib()
-    lib.tccl_ag_gemm_param_bytes.restype = C.c_uint64
-    lib.tccl_ag_gemm_pair_param_bytes.restype = C.c_uint64
     grid = _gemm_ctas(w, pair)
     if comm_ctas <= 0:
         # Few data movers: every mover CTA is an SM the GEMM does not get, and 8 movers
@@ -279,57 +311,37 @@ def all_gather_gemm(a_shard, bt, a_full=None, out=None, *, comm_ctas: int = 0, s
         # Llama-3-8B up-projection: 8 movers 116 us, 16: 121 us, 24: 125 us, 48: 128 us).
         comm_ctas = w.config.ag_movers if grid > 16 else 2
         comm_ctas = max(1, min(comm_ctas, grid - 1))
-    outs = {}
-    Os = _locals(w, out) if out is not None else None
-    arr = (L.AgGemmArgs * len(w.local_ranks))()
-    for i, r in enumerate(w.local_ranks):
-        ar, br = As[r], Bs[r]
+    arr = (L.AgGemmArgs * len(As))()
+    for i, (r, ar, br) in enumerate(zip(w.local_ranks, As, Bs)):
         if ar.stride(1) != 1 or br.stride(1) != 1:
             raise ValueError("operands must have a unit inner stride")
-        o = Os[r] if Os is not None else torch.empty((M, n_out), dtype=torch.bfloat16, device=ar.device)
-        if o.shape != (M, n_out) or o.dtype != torch.bfloat16 or o.stride(1) != 1:
-            raise ValueError(f"out must be bf16 [{M}, {n_out}] with a unit inner stride")
-        outs[r] = o
-        g = L.AgGemmArgs()
+        optr, ldo = 0, n_out
+        if Os is not None:
+            o = Os[i]
+            if o.shape != (M, n_out) or o.dtype != torch.bfloat16 or o.stride(1) != 1:
+                raise ValueError(f"out must be bf16 [{M}, {n_out}] with a unit inner stride")
+            optr, ldo = o.data_ptr(), o.stride(0)
+        g = arr[i]
         g.a_shard = ar.data_ptr()
         for q, v in enumerate(full_ptrs):
             g.a_full[q] = v
         g.mc_a_full = mc
-        g.bt, g.out = br.data_ptr(), o.data_ptr()
+        g.bt, g.out = br.data_ptr(), optr
         g.m, g.n, g.k = M, N, Kd
-        g.lda_shard, g.lda_full, g.ldb, g.ldo = ar.stride(0), Kd, br.stride(0), o.stride(0)
+        g.lda_shard, g.lda_full, g.ldb, g.ldo = ar.stride(0), Kd, br.stride(0), ldo
         g.comm_ctas = max(1, int(w.config.ag_batches)) if pair else comm_ctas  # pair kernel: batches of the mover phase
         g.swiglu = 1 if swiglu else 0
-        g.trace = _trace_ptr(w, trace, r, grid)
-        g.lsu_movers = int(lsu_movers)
+        g.lsu_movers = lsu_movers
         if pair:  # bits: 2 = move the shard only (timeline tool), 4 = movers send destination by destination
-            g.lsu_movers = (2 if int(lsu_movers) == 2 else 0) | (4 if w.config.ag_ring else 0)
+            g.lsu_movers = (2 if lsu_movers == 2 else 0) | (4 if w.config.ag_ring else 0)
         if pair and w.config.ag_schedule and W > 1:
             nb = max(1, min(int(w.config.ag_batches), rows // 128))
             sched = _ag_sched_tensor(w, r, rows // 128, -(-N // 256), grid // 2, nb, Kd, True, ar.device)
             g.sched, g.sched_stride = sched.data_ptr(), sched.shape[1]
-        arr[i] = g
-    stream = torch.cuda.current_stream(a0.device).cuda_stream
-    if pair:
-        fn = lib.tccl_allgather_gemm_pair
-        extra = (C.c_uint64(half_bytes),)
-    else:
-        fn = lib.tccl_allgather_gemm
-        extra = ()
-    if w.plans is not None:
-        l = L.Launch(grid, 256, 0, 0, C.c_void_p(stream))
-        rc = fn(C.byref(w.comm), C.byref(arr[0]), None, *extra, C.byref(l))
-    else:
-        pb = int(lib.tccl_ag_gemm_pair_param_bytes() if pair else lib.tccl_ag_gemm_param_bytes())
-        scratch = torch.empty(pb * W + 64, dtype=torch.uint8, device=a0.device)
-        base = (scratch.data_ptr() + 63) & ~63
-        w._keep.append(scratch)
-        l = L.Launch(grid, 256, W, 0, C.c_void_p(stream))
-        rc = fn(C.c_void_p(w.comms_dev.data_ptr()), arr, C.c_void_p(base), *extra, C.byref(l))
-    L.check(rc, "tccl_allgather_gemm_pair" if pair else "tccl_allgather_gemm")
-    w.launches += 1
-    res = out if out is not None else ([outs[r] for r in w.local_ranks] if w.plans is None else outs[w.local_ranks[0]])
-    return res, ret_full
+    p = FusedPlan(w, "tccl_allgather_gemm_pair" if pair else "tccl_allgather_gemm", arr, grid, 256,
+                  (C.c_uint64(half_bytes),) if pair else (), ((M, n_out), (n_out, 1)), "ag_gemm_pair" if pair else "ag_gemm")
+    p.views = views
+    return p
 
 
 def all_reduce_bias_residual_rmsnorm(x, weight, bias=None, residual=None, eps: float = 1e-5, out=None,
@@ -344,6 +356,20 @@ def all_reduce_bias_residual_rmsnorm(x, weight, bias=None, residual=None, eps: f
     they are allocated and cached per shape when omitted (pass ``residual_out=True``
     to ask for the pre-norm sum).  Returns ``y`` or ``(y, residual_out)``."""
     w = get_world(world)
+    want_res = residual_out is not None and residual_out is not False
+    given = residual_out if want_res and residual_out is not True else None
+    Ws, Bs, Rs = _locals(w, weight), (_locals(w, bias) if bias is not None else None), \
+        (_locals(w, residual) if residual is not None else None)
+    key = ("arn", w.tkey(x), _tkeys(Ws), Bs and _tkeys(Bs), Rs and _tkeys(Rs), eps, None if out is None else w.tkey(out),
+           want_res, None if given is None else w.tkey(given), algo)
+    p = _planned(w, key, _plan_arn, x, Ws, Bs, Rs, eps, out, want_res, given, algo)
+    p.go(w, Ws[0].device)
+    if out is None:
+        out = p.views[0]
+    return (out, p.views[1] if given is None else given) if want_res else out
+
+
+def _plan_arn(w, x, Ws, Bs, Rs, eps, out, want_res, given_res, algo) -> FusedPlan:
     check_sym_tensor(w, x, "input")
     x0 = w.local(x, w.local_ranks[0])
     if x0.dim() != 2:
@@ -356,7 +382,7 @@ def all_reduce_bias_residual_rmsnorm(x, weight, bias=None, residual=None, eps: f
     cache = w.__dict__.setdefault("_arn_buffers", {})
 
     def sym(tag, given):
-        if given is not None and given is not True:
+        if given is not None:
             check_sym_tensor(w, given, tag)
             return given
         key = (tag, T, H, x0.dtype)
@@ -364,20 +390,17 @@ def all_reduce_bias_residual_rmsnorm(x, weight, bias=None, residual=None, eps: f
             cache[key] = w.empty((T, H), x0.dtype)
         return cache[key]
 
+    o_given = out is not None
     out = sym("out", out)
-    want_res = residual_out is not None and residual_out is not False
-    res_out = sym("residual_out", residual_out) if want_res else None
+    res_out = sym("residual_out", given_res) if want_res else None
     if algo == "auto":
         algo = "nvls" if w.has_nvls and w.world_size > 2 else "p2p"
     if algo == "nvls" and not w.has_nvls:
         raise RuntimeError("nvls variant needs NVLS multicast")
-    Ws, Bs, Rs = _locals(w, weight), (_locals(w, bias) if bias is not None else None), \
-        (_locals(w, residual) if residual is not None else None)
     xp, op = w.peer_ptrs(x), w.peer_ptrs(out)
     rp = w.peer_ptrs(res_out) if want_res else None
-    args = {}
-    for r in w.local_ranks:
-        a = L.ArnArgs()
+    arr = (L.ArnArgs * len(w.local_ranks))()
+    for i, a in enumerate(arr):
         for q in range(w.world_size):
             a.x[q], a.out[q] = xp[q], op[q]
             a.res_out[q] = rp[q] if rp else 0
@@ -385,9 +408,8 @@ def all_reduce_bias_residual_rmsnorm(x, weight, bias=None, residual=None, eps: f
         a.mc_res_out = w.mc_ptr(res_out) if want_res else 0
         for name, src in (("weight", Ws), ("bias", Bs), ("residual", Rs)):
             if src is None:
-                setattr(a, name, 0)
                 continue
-            tns = src[r]
+            tns = src[i]
             if tns.dtype != x0.dtype or not tns.is_contiguous() or tns.data_ptr() % 16:
                 raise ValueError(f"{name} must be contiguous, 16-byte aligned and of x's dtype")
             if tns.numel() != (T * H if name == "residual" else H):
@@ -395,27 +417,15 @@ def all_reduce_bias_residual_rmsnorm(x, weight, bias=None, residual=None, eps: f
             setattr(a, name, tns.data_ptr())
         a.eps, a.tokens, a.hidden, a.dtype = float(eps), T, H, dt
         a.flags = w.coll_flags()
-        args[r] = a
     rows = -(-T // w.world_size)
     nv = H // vpt
-    per_sm = 2 if nv <= 512 and w.plans is not None else 1  # narrow rows: two CTAs per SM
-    batch = 1                                                # rows a CTA handles together (kernel's R)
+    per_sm = 2 if nv <= 512 and not w.emulated else 1  # narrow rows: two CTAs per SM
+    batch = 1                                          # rows a CTA handles together (kernel's R)
     grid = max(1, min(-(-rows // batch), w.max_ctas() * per_sm, K["TCCL_MAX_BLOCKS"]))
-    fn = L.lib().tccl_allreduce_bias_residual_rmsnorm
-    nvls = 1 if algo == "nvls" else 0
-    stream = torch.cuda.current_stream(x0.device).cuda_stream
-    if w.plans is not None:
-        l = L.Launch(grid, 512, 0, dt, C.c_void_p(stream))
-        rc = fn(C.byref(w.comm), C.byref(args[w.local_ranks[0]]), nvls, H, C.byref(l))
-    else:
-        arr = (L.ArnArgs * w.world_size)(*[args[r] for r in w.local_ranks])
-        dev = w._to_device(arr)
-        w._keep.append(dev)
-        l = L.Launch(grid, 512, w.world_size, dt, C.c_void_p(stream))
-        rc = fn(C.c_void_p(w.comms_dev.data_ptr()), C.c_void_p(dev.data_ptr()), nvls, H, C.byref(l))
-    L.check(rc, "tccl_allreduce_bias_residual_rmsnorm")
-    w.launches += 1
-    return (out, res_out) if want_res else out
+    p = FusedPlan(w, "tccl_allreduce_bias_residual_rmsnorm", arr, grid, 512, (1 if algo == "nvls" else 0,))
+    # only the communicator's own buffers are kept (it keeps them anyway), never the caller's
+    p.views = (None if o_given else out, None if given_res is not None else res_out)
+    return p
 
 
 def pack_gate_up(gate_w: torch.Tensor, up_w: torch.Tensor) -> torch.Tensor:

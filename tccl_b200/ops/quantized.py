@@ -19,7 +19,8 @@ import torch
 from ..parallel.world import WorldBase
 from ..utils import lib as L
 from ._common import get_world
-from .fused import _locals, _stage_handoff
+from .collectives import Plan, _planned
+from .fused import _locals, _stage_handoff, _tkeys
 
 __all__ = ["quantized_all_reduce", "QUANT_CHUNK"]
 
@@ -34,9 +35,17 @@ def quantized_all_reduce(x, out=None, *, world: Optional[WorldBase] = None):
     """Sum ``x`` (bf16, any device memory, ``numel % 2048 == 0``) over all ranks with fp8 on the
     wire; returns a bf16 tensor (``out`` or a new one).  ``out`` may be ``x`` itself."""
     w = get_world(world)
-    W = w.world_size
     xs = _locals(w, x)
-    x0 = xs[w.local_ranks[0]]
+    os_ = _locals(w, out) if out is not None else None
+    p = _planned(w, ("fp8wire", _tkeys(xs), os_ and _tkeys(os_)), _plan_quantized, xs, os_)
+    _stage_handoff(w, "fp8wire")
+    res = p.run()
+    return out if out is not None else res
+
+
+def _plan_quantized(w, xs, os_) -> Plan:
+    W = w.world_size
+    x0 = xs[0]
     if x0.dtype != torch.bfloat16:
         raise TypeError("quantized_all_reduce takes bfloat16 tensors")
     n = x0.numel()
@@ -48,19 +57,16 @@ def quantized_all_reduce(x, out=None, *, world: Optional[WorldBase] = None):
     have = (w.config.stage_mb << 20) - w.ll_bytes
     if need > have:
         raise ValueError(f"staging area too small: need {need >> 20} MiB, have {have >> 20} MiB (raise TCCL_STAGE_MB)")
-    outs = {}
-    os_ = _locals(w, out) if out is not None else None
     args = {}
-    for r in w.local_ranks:
-        o = os_[r] if os_ is not None else torch.empty_like(xs[r])
-        if o.dtype != torch.bfloat16 or o.numel() != n or not o.is_contiguous() or o.data_ptr() % 16:
-            raise ValueError("out must be a contiguous, 16-byte aligned bf16 tensor of the input's size")
-        outs[r] = o
-        args[r] = QarArgs(xs[r].data_ptr(), o.data_ptr(), n, 0)
-    _stage_handoff(w, "fp8wire")
+    for i, r in enumerate(w.local_ranks):
+        optr = 0
+        if os_ is not None:
+            o = os_[i]
+            if o.dtype != torch.bfloat16 or o.numel() != n or not o.is_contiguous() or o.data_ptr() % 16:
+                raise ValueError("out must be a contiguous, 16-byte aligned bf16 tensor of the input's size")
+            optr = o.data_ptr()
+        args[r] = QarArgs(xs[i].data_ptr(), optr, n, 0)
     cps = -(-(n // QUANT_CHUNK) // W)
     grid = max(1, min(-(-cps // 8), 2 * w.max_ctas()))  # a CTA's 8 warps take 8 chunks at a time
-    w.launch("tccl_allreduce_fp8wire", args, grid, 256)
-    if out is not None:
-        return out
-    return w.wrap(outs)
+    go = w.prepare("tccl_allreduce_fp8wire", args, grid, 256)
+    return Plan(w, go, args, fresh=None if os_ is not None else (tuple(x0.shape), x0.dtype, x0.device))

@@ -32,7 +32,7 @@ from ..parallel.tree import tree_neighbours
 from ..parallel.world import WorldBase
 from ..utils import lib as L
 from ._common import K, check_sym_tensor, dtype_code, get_world
-from .collectives import _OUT, _X, Plan, _cached, _check_out, _key
+from .collectives import _OUT, _X, Plan, _check_out, _planned
 
 __all__ = ["double_tree_all_reduce"]
 
@@ -59,9 +59,8 @@ def _tree_grid(w: WorldBase, nbytes: int):
 
 def double_tree_all_reduce(tensor, out=None, *, inplace: bool = False, world: Optional[WorldBase] = None):
     w = get_world(world)
-    cfg = w.config  # the settings that shape the plan are part of its key
-    knobs = (cfg.tree_ll_max_bytes, cfg.tree_pull_min_bytes, cfg.tree_ctas, cfg.tree_chunk_bytes)
-    return _cached(w, _key("tree", w, tensor, out, inplace, knobs), lambda: _plan(w, tensor, out, inplace), tensor, out)
+    key = ("tree", w.tkey(tensor), None if out is None else w.tkey(out), inplace)
+    return _planned(w, key, _plan, tensor, out, inplace).run(tensor, out)
 
 
 def _plan(w: WorldBase, x, out, inplace: bool) -> Plan:
@@ -117,7 +116,7 @@ def _plan(w: WorldBase, x, out, inplace: bool) -> Plan:
     if inplace:
         return Plan(w, go, args, result=_X)
     shape, dtype, dev = tuple(x0.shape), x0.dtype, x0.device
-    return Plan(w, go, args, alloc=lambda r: torch.empty(shape, dtype=dtype, device=dev))
+    return Plan(w, go, args, fresh=(shape, dtype, dev))
 
 
 def _neighbours(a, W: int, r: int) -> None:
@@ -165,4 +164,4 @@ def _plan_ll(w: WorldBase, x, out, inplace: bool, x0, dt: int, nbytes: int) -> P
     if inplace:
         return Plan(w, go, args, result=_X)
     shape, dtype, dev = tuple(x0.shape), x0.dtype, x0.device
-    return Plan(w, go, args, alloc=lambda r: torch.empty(shape, dtype=dtype, device=dev))
+    return Plan(w, go, args, fresh=(shape, dtype, dev))

@@ -18,7 +18,7 @@ import torch
 
 from ..config import Config
 from ..utils import lib as L
-from .world import WorldBase, _status_dict, tree_ring_bytes
+from .world import PlanCache, WorldBase, _status_dict, tree_ring_bytes
 
 K = L.K
 
@@ -51,11 +51,17 @@ class EmuTensor:
     def numel(self):
         return self.parts[0].numel()
 
+    def half(self, i: int) -> "EmuTensor":
+        """Entry ``i`` of every rank's leading dimension."""
+        return EmuTensor([p[i] for p in self.parts])
+
     def view_all(self, fn) -> "EmuTensor":
         return EmuTensor([fn(p) for p in self.parts])
 
 
 class EmuWorld(WorldBase):
+    emulated = True
+
     def __init__(self, world_size: int, config: Optional[Config] = None, device="cuda:0"):
         if not torch.cuda.is_available():
             raise RuntimeError("EmuWorld needs a CUDA device")
@@ -65,6 +71,8 @@ class EmuWorld(WorldBase):
         self.world_size = world_size
         self.config = config or Config.from_env()
         self.device = torch.device(device)
+        if self.device.index is None:
+            self.device = torch.device("cuda", torch.cuda.current_device())
         W = world_size
         self._flag_words = K["TCCL_FLAG_WORDS"]
         self._stage_bytes = int(self.config.stage_mb) << 20
@@ -76,22 +84,19 @@ class EmuWorld(WorldBase):
         self._zero_tree_ll()
         self.local_states = [torch.zeros(K["TCCL_LOCAL_WORDS"], dtype=torch.int32, device=self.device) for _ in range(W)]
         self.ll_bytes = min(2 << 20, self._stage_bytes // 4)
-        self._keep = []
-        self.plans = None  # emulated launches are not cached
-        self._upload_comms()
+        self.plans = PlanCache(self.config.plan_cache_size)
+        self.comms = (L.Comm * W)()  # host structs: they travel with every launch
+        self._fill_comms()
 
     def _zero_tree_ll(self):
         """The small-message tree slots must not start out with bits that look like a flag."""
         for s in self.stages:
             s[self._stage_bytes: self._stage_bytes + K["TCCL_TREE_LL_BYTES"]].zero_()
 
-    def _upload_comms(self):
-        W = self.world_size
-        arr = (L.Comm * W)()
-        for r in range(W):
-            c = arr[r]
-            c.world, c.rank = W, r
-            for p in range(W):
+    def _fill_comms(self):
+        for r, c in enumerate(self.comms):
+            c.world, c.rank = self.world_size, r
+            for p in range(self.world_size):
                 c.flags[p] = self.flags[p].data_ptr()
                 c.stage[p] = self.stages[p].data_ptr()
             c.mc_flags = 0
@@ -101,12 +106,6 @@ class EmuWorld(WorldBase):
             c.timeout_ns = self.config.timeout_ns
             c.ll_bytes = self.ll_bytes
             c.tree_bytes = self.tree_bytes
-        self._comms_host = arr
-        self.comms_dev = self._to_device(arr)
-
-    def _to_device(self, cstruct_array) -> torch.Tensor:
-        raw = bytes(cstruct_array)
-        return torch.frombuffer(bytearray(raw), dtype=torch.uint8).to(self.device)
 
     # -- tensors
     def empty(self, shape, dtype=torch.bfloat16) -> EmuTensor:
@@ -136,7 +135,11 @@ class EmuWorld(WorldBase):
         return x.parts[r]
 
     def wrap(self, per_rank):
-        return EmuTensor([per_rank[r] for r in range(self.world_size)])
+        return EmuTensor(per_rank)
+
+    def tkey(self, x: EmuTensor) -> tuple:
+        x0 = x.parts[0]
+        return (tuple([p.data_ptr() for p in x.parts]), x0.shape, x0.stride(), x0.dtype)
 
     def stage_ptrs(self) -> List[int]:
         return [s.data_ptr() for s in self.stages]
@@ -164,28 +167,27 @@ class EmuWorld(WorldBase):
 
     def prepare(self, name, args_by_rank, grid, block, dtype_code=0):
         W = self.world_size
-        first = args_by_rank[0]
         fn = getattr(L.lib(), name)
+        # one contiguous array for the launcher; the caller's dict holds views of it from here on
+        arr = (type(args_by_rank[0]) * W)(*[args_by_rank[r] for r in range(W)])
+        for r in range(W):
+            args_by_rank[r] = arr[r]
         l = L.Launch(int(grid), int(block), W, int(dtype_code), None)
-        comms = C.c_void_p(self.comms_dev.data_ptr())
+        comms_ref, arr_ref, l_ref = self.comm_ref(), C.byref(arr), C.byref(l)
+        raw_stream = torch._C._cuda_getCurrentRawStream
+        dev = self.device.index
 
         def go():
-            # the structs may have been patched since the last call: upload them again
-            arr = (type(first) * W)()
-            for r in range(W):
-                C.memmove(C.byref(arr[r]), C.byref(args_by_rank[r]), C.sizeof(first))
-            args_dev = self._to_device(arr)
-            self._keep.append(args_dev)
-            if len(self._keep) > 64:
-                torch.cuda.synchronize(self.device)
-                del self._keep[:-1]
-            l.stream = torch.cuda.current_stream(self.device).cuda_stream
-            rc = fn(comms, C.c_void_p(args_dev.data_ptr()), C.byref(l))
+            l.stream = raw_stream(dev)
+            rc = fn(comms_ref, arr_ref, l_ref)
             if rc:
                 L.check(rc, name)
             self.launches += 1
 
         return go
+
+    def comm_ref(self):
+        return C.byref(self.comms)
 
     # -- state
     def last_status(self, rank: int = None):
@@ -213,5 +215,4 @@ class EmuWorld(WorldBase):
 
     def set_timeout_ms(self, ms: float) -> None:
         self.config.timeout_ms = ms
-        torch.cuda.synchronize(self.device)
-        self._upload_comms()
+        self._fill_comms()

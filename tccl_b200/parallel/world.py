@@ -80,6 +80,7 @@ class WorldBase:
     config: Config
     device: torch.device
     launches: int = 0  # kernels of this library launched so far
+    emulated: bool = False  # all ranks in this process, on one GPU
 
     # -- to be provided by subclasses
     @property
@@ -99,15 +100,26 @@ class WorldBase:
     def local(self, x, r: int) -> torch.Tensor:
         raise NotImplementedError
 
-    def wrap(self, per_rank: Dict[int, torch.Tensor]):
-        """Turn {rank: tensor} into what this world hands back to the user."""
+    def tkey(self, x) -> tuple:
+        """What identifies a (symmetric or ordinary) tensor argument in a plan's key: address, extent AND
+        layout — a strided view that shares address, element count and dtype with a contiguous tensor
+        must not hit that tensor's plan."""
+        return (x.data_ptr(), x.shape, x.stride(), x.dtype)
+
+    def wrap(self, per_rank: List[torch.Tensor]):
+        """Turn the local ranks' tensors into what this world hands back to the user."""
         raise NotImplementedError
 
     def prepare(self, name: str, args_by_rank: Dict[int, C.Structure], grid: int, block: int,
                 dtype_code: int = 0):
         """Bind one kernel launch to its arguments; returns a zero-argument callable
-        that enqueues it on the current stream.  The argument structs stay owned by
-        the caller, who may patch a field (an output pointer) between calls."""
+        that enqueues it on the current stream.  The caller may patch a field (an output
+        pointer) of ``args_by_rank``'s structs between calls; a world may replace the dict's
+        values by structs of its own, so they are looked up there again."""
+        raise NotImplementedError
+
+    def comm_ref(self):
+        """The communicator struct(s) as the native launchers take them."""
         raise NotImplementedError
 
     def launch(self, name: str, args_by_rank: Dict[int, C.Structure], grid: int, block: int,
@@ -272,7 +284,7 @@ class RealWorld(WorldBase):
         return x
 
     def wrap(self, per_rank):
-        return per_rank[self.rank]
+        return per_rank[0]
 
     def stage_ptrs(self) -> List[int]:
         return self._stage_ptrs
@@ -311,6 +323,9 @@ class RealWorld(WorldBase):
 
         go.keep = (a, l)  # the structs the references point into
         return go
+
+    def comm_ref(self):
+        return C.byref(self.comm)
 
     # -- state
     def last_status(self) -> dict:
