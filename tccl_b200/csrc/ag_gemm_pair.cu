@@ -42,6 +42,8 @@ struct alignas(64) AgGemmPairParams {
   __nv_bfloat16* out;
   int lda_shard, lda_full, ldo;
   int tiles_n, tiles_m_per_rank;
+  Raster raster;         // order of the rank's own tiles
+  TailSplitSchedule tail;  // one rank: the units of a pair
   int swiglu;
   const int32_t* sched;  // optional: every pair's tiles in running order (see tccl_ag_gemm_args)
   int sched_stride;
@@ -74,11 +76,17 @@ struct AgGemmPairPolicy {
     const int t = pair + i * npairs;
     const int tm2 = p->tiles_m_per_rank / 2, tn = p->tiles_n, W = c->world;
     const int own = tm2 * tn;
+    if (W == 1) {  // all rows are here: whole waves, then half tiles
+      if (!p->tail.unit(pair, i, mt, half)) return false;
+      p->raster.at(mt, mt, nt);
+      mt *= 2;
+      return true;
+    }
     half = 0;
     if (t >= W * own) return false;
     if (t < own) {  // own rows first: no waiting
-      mt = c->rank * p->tiles_m_per_rank + 2 * (t / tn);
-      nt = t % tn;
+      p->raster.at(t, mt, nt);
+      mt = c->rank * p->tiles_m_per_rank + 2 * mt;
       return true;
     }
     const int u = t - own;
@@ -254,49 +262,35 @@ struct AgGemmPairPolicy {
     }
   }
   __device__ __forceinline__ bool epilogue(int mt, int nt, int col_lo, int ncols, uint32_t taddr, int quad, int lane,
-                                           const Abort&, const Smem2&) const {
-    const int row = mt * 128 + quad * 32 + lane;
-    __nv_bfloat16* crow = p->out + (size_t)row * p->ldo;
+                                           const Abort&, const Smem2& sm) const {
+    const int row0 = mt * 128 + quad * 32;
+    uint8_t* buf = sm.epi[0] + quad * 4096;
     if (p->swiglu) {
       // every 256-wide tile holds 128 gate columns followed by the 128 matching up columns; a half
       // tile's accumulator holds 64 of each (see b_tile)
-      const int hw = ncols / 2;
+      const int hw = ncols / 2, col = nt * (BN2 / 2) + col_lo / 2;
 #pragma unroll 1
-      for (int cg = 0; cg < hw / 32; ++cg) {
-        uint32_t g[32], u[32];
-        tmem_ld_32x32(taddr + cg * 32, g);
-        tmem_ld_32x32(taddr + hw + cg * 32, u);
-        tmem_ld_wait();
-        const int col0 = nt * (BN2 / 2) + col_lo / 2 + cg * 32;
-        if (row < p->shp.M) {
+      for (int c = 0; c < hw; c += 64) {
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          uint32_t g[32], u[32];
+          tmem_ld_32x32(taddr + c + h * 32, g);
+          tmem_ld_32x32(taddr + hw + c + h * 32, u);
+          tmem_ld_wait();
 #pragma unroll
           for (int v = 0; v < 4; ++v) {
-            if (col0 + v * 8 < p->shp.N / 2) {
-              uint32_t o[8];
+            uint32_t o[8];
 #pragma unroll
-              for (int e = 0; e < 8; ++e) {
-                const float gv = __uint_as_float(g[v * 8 + e]), uv = __uint_as_float(u[v * 8 + e]);
-                o[e] = __float_as_uint(gv / (1.f + __expf(-gv)) * uv);
-              }
-              st_local(crow + col0 + v * 8, pack8_bf16(o));
-            }
+            for (int e = 0; e < 8; ++e) o[e] = __float_as_uint(swiglu(__uint_as_float(g[v * 8 + e]), __uint_as_float(u[v * 8 + e])));
+            stage_put(buf, lane, h * 4 + v, pack8_bf16(o));
           }
         }
+        stage_flush(buf, lane, p->out + (size_t)row0 * p->ldo + col + c, p->ldo, p->shp.M - row0, p->shp.N / 2 - col - c);
       }
       return true;
     }
-#pragma unroll 1
-    for (int cg = 0; cg < ncols / 32; ++cg) {  // a half tile's 128 columns sit at the start of the accumulator
-      uint32_t r[32];
-      tmem_ld_32x32(taddr + cg * 32, r);
-      tmem_ld_wait();
-      const int col0 = nt * BN2 + col_lo + cg * 32;
-      if (row < p->shp.M) {
-#pragma unroll
-        for (int v = 0; v < 4; ++v)
-          if (col0 + v * 8 < p->shp.N) st_local(crow + col0 + v * 8, pack8_bf16(r + v * 8));
-      }
-    }
+    // a half tile's 128 columns sit at the start of the accumulator
+    store_rows(buf, p->out, p->ldo, row0, p->shp.M, nt * BN2 + col_lo, p->shp.N, ncols, taddr, lane);
     return true;
   }
 };
@@ -347,7 +341,8 @@ ag_gemm_pair_kernel_emu(const __grid_constant__ EmuParams<AgGemmPairParams> e) {
   ag_gemm_pair_body(e.comm[blockIdx.y], e.args[blockIdx.y], blockIdx.x, gridDim.x);
 }
 
-static int fill_params(AgGemmPairParams* p, const tccl_ag_gemm_args* g, int world, int rank, uint64_t half_bytes) {
+static int fill_params(AgGemmPairParams* p, const tccl_ag_gemm_args* g, int world, int rank, int pairs,
+                       uint64_t half_bytes) {
   if (g->m <= 0 || g->n <= 0 || g->k <= 0) return -TCCL_EINVAL;
   if ((g->lda_shard % 8) || (g->lda_full % 8) || (g->ldb % 8) || (g->ldo % 8) || (g->k % 8) || (g->n % 8))
     return -TCCL_EALIGN;
@@ -380,6 +375,8 @@ static int fill_params(AgGemmPairParams* p, const tccl_ag_gemm_args* g, int worl
   p->ldo = g->ldo;
   p->tiles_n = (g->n + BN2 - 1) / BN2;
   p->tiles_m_per_rank = rows / 128;
+  p->raster = Raster{p->tiles_n, raster_group(rows / 256, g->k), rows / 256};
+  p->tail.init(rows / 256 * p->tiles_n, pairs);
   p->swiglu = g->swiglu;
   p->batches = g->comm_ctas > 0 ? g->comm_ctas : 2;
   p->movers_only = (g->lsu_movers & 2) != 0;
@@ -416,7 +413,7 @@ extern "C" int tccl_allgather_gemm_pair(const tccl_comm* comm, const tccl_ag_gem
   }
   if (l->n_emu == 0) {
     AgGemmPairParams p;
-    int rc = fill_params(&p, args, comm->world, comm->rank, half_bytes);
+    int rc = fill_params(&p, args, comm->world, comm->rank, l->grid / 2, half_bytes);
     if (rc) return rc;
     ag_gemm_pair_kernel<<<l->grid, kThreads, kSmem2, s>>>(*comm, p);
     return (int)cudaGetLastError();
@@ -425,7 +422,7 @@ extern "C" int tccl_allgather_gemm_pair(const tccl_comm* comm, const tccl_ag_gem
   if (W < 1 || W > TCCL_MAX_WORLD) return -TCCL_EINVAL;
   tccl::EmuParams<AgGemmPairParams> ep;
   for (int r = 0; r < W; ++r) {
-    int rc = fill_params(&ep.args[r], &args[r], W, r, half_bytes);
+    int rc = fill_params(&ep.args[r], &args[r], W, r, l->grid / 2, half_bytes);
     if (rc) return rc;
     ep.comm[r] = comm[r];
   }

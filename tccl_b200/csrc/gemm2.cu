@@ -7,61 +7,17 @@
 namespace tccl {
 namespace gemm2 {
 
-// Tile order of a persistent grid of `pairs` CTA pairs over `total` 256 x 256 tiles: the
-// whole waves first (tile = pair + i * pairs), then the tiles of the last, partial wave cut
-// into left and right halves, so that the tail costs every pair at most half a tile more
-// than the pairs that are done.
-struct TailSplitSchedule {
-  int total, pairs, nfull, rem;
-  __host__ __device__ void init(int total_, int pairs_) {
-    total = total_;
-    pairs = pairs_;
-    nfull = (total / pairs) * pairs;
-    rem = total - nfull;
-  }
-  __device__ __forceinline__ bool unit(int pair, int i, int& tile, int& half) const {
-    const int u = pair + i * pairs;
-    if (u < nfull) {
-      tile = u;
-      half = 0;
-      return true;
-    }
-    const int h = u - nfull;
-    if (h >= 2 * rem) return false;
-    tile = nfull + (h >> 1);
-    half = 1 + (h & 1);
-    return true;
-  }
-};
-
-// epilogue shared by the plain kernel: tensor memory -> registers -> bf16 rows of C
-__device__ __forceinline__ void store_rows(__nv_bfloat16* crow, bool row_ok, int N, int col_base, int ncols, uint32_t taddr) {
-#pragma unroll 1
-  for (int c = 0; c < ncols / 32; ++c) {
-    uint32_t r[32];
-    tmem_ld_32x32(taddr + c * 32, r);
-    tmem_ld_wait();
-    const int col = col_base + c * 32;
-    if (row_ok) {
-#pragma unroll
-      for (int v = 0; v < 4; ++v)
-        if (col + v * 8 < N) st_local(crow + col + v * 8, pack8_bf16(r + v * 8));
-    }
-  }
-}
-
 struct PlainPolicy2 {
   const CUtensorMap *map_a, *map_b128, *map_b64;
   __nv_bfloat16* C;
   int M, N, ldc;
-  int tiles_n;
+  Raster raster;
   TailSplitSchedule sched;
   __device__ __forceinline__ bool tile(int i, int& mt, int& nt, int& half) const {
     int t;
     if (!sched.unit(blockIdx.x >> 1, i, t, half)) return false;
-    const int mt2 = t / tiles_n;
-    nt = t - mt2 * tiles_n;
-    mt = 2 * mt2;
+    raster.at(t, mt, nt);
+    mt *= 2;
     return true;
   }
   __device__ __forceinline__ void b_tile(int nt, int half, int cta, const CUtensorMap*& map, int& y) const {
@@ -77,31 +33,25 @@ struct PlainPolicy2 {
   __device__ __forceinline__ void between_tiles(int, int, const Abort&) const {}
   __device__ __forceinline__ void epilogue_begin(int, int, const Abort&) const {}
   __device__ __forceinline__ bool epilogue(int mt, int nt, int col0, int ncols, uint32_t taddr, int quad, int lane,
-                                           const Abort&, const Smem2&) const {
-    const int row = mt * 128 + quad * 32 + lane;
-    store_rows(C + (size_t)row * ldc, row < M, N, nt * BN2 + col0, ncols, taddr);
+                                           const Abort&, const Smem2& sm) const {
+    store_rows(sm.epi[0] + quad * 4096, C, ldc, mt * 128 + quad * 32, M, nt * BN2 + col0, N, ncols, taddr, lane);
     return true;
   }
 };
 
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b128,
-                 const __grid_constant__ CUtensorMap map_b64, const Shape shp, PlainPolicy2 pol, uint32_t* status) {
+                 const __grid_constant__ CUtensorMap map_b64, const Shape shp, PlainPolicy2 pol, uint32_t* status,
+                 uint64_t timeout_ns, uint64_t* trace) {
   tccl_comm fake;
   fake.local = status ? status - TCCL_LOCAL_STATUS : nullptr;
   pol.map_a = &map_a;
   pol.map_b128 = &map_b128;
   pol.map_b64 = &map_b64;
-  run_mainloop2(shp, pol, status ? &fake : nullptr, 2000000000ull);
+  run_mainloop2(shp, pol, status ? &fake : nullptr, timeout_ns, trace ? trace + (size_t)blockIdx.x * 64 : nullptr);
 }
 
-}  // namespace gemm2
-}  // namespace tccl
-
-using namespace tccl::gemm;
-using namespace tccl::gemm2;
-
-extern "C" int tccl_gemm_bf16_pair(const tccl_gemm_args* g, int grid, void* stream) {
+int launch_gemm_pair(const tccl_gemm_args* g, int grid, cudaStream_t stream, uint64_t timeout_ns, uint64_t* trace) {
   if (!g || g->m <= 0 || g->n <= 0 || g->k <= 0) return -TCCL_EINVAL;
   if ((g->lda % 8) || (g->ldb % 8) || (g->ldc % 8) || (g->n % 8) || (g->k % 8)) return -TCCL_EALIGN;
   if (((uintptr_t)g->a | (uintptr_t)g->bt | (uintptr_t)g->c) & 15) return -TCCL_EALIGN;
@@ -117,11 +67,12 @@ extern "C" int tccl_gemm_bf16_pair(const tccl_gemm_args* g, int grid, void* stre
   pol.M = g->m;
   pol.N = g->n;
   pol.ldc = g->ldc;
-  pol.tiles_n = (g->n + BN2 - 1) / BN2;
-  const int total = ((g->m + 255) / 256) * pol.tiles_n;
+  const int tm = (g->m + 255) / 256, tn = (g->n + BN2 - 1) / BN2, total = tm * tn;
+  pol.raster = Raster{tn, raster_group(tm, g->k), tm};
   if (grid <= 0) grid = tccl_num_sms();
   grid &= ~1;
-  if (grid > 2 * total) grid = 2 * total;
+  // fewer tiles than pairs: half tiles if every half then has a pair of its own, else one whole tile each
+  if (grid > 2 * total) grid = grid >= 4 * total ? 4 * total : 2 * total;
   if (grid < 2) return -TCCL_EINVAL;
   pol.sched.init(total, grid / 2);
   static bool attr_set = false;
@@ -131,7 +82,14 @@ extern "C" int tccl_gemm_bf16_pair(const tccl_gemm_args* g, int grid, void* stre
     attr_set = true;
   }
   Shape shp{g->m, g->n, g->k};
-  gemm_pair_kernel<<<grid, kThreads, kSmem2, reinterpret_cast<cudaStream_t>(stream)>>>(
-      ma, mb128, mb64, shp, pol, reinterpret_cast<uint32_t*>(g->status));
+  gemm_pair_kernel<<<grid, kThreads, kSmem2, stream>>>(ma, mb128, mb64, shp, pol, reinterpret_cast<uint32_t*>(g->status),
+                                                       timeout_ns, trace);
   return (int)cudaGetLastError();
+}
+
+}  // namespace gemm2
+}  // namespace tccl
+
+extern "C" int tccl_gemm_bf16_pair(const tccl_gemm_args* g, int grid, void* stream) {
+  return tccl::gemm2::launch_gemm_pair(g, grid, reinterpret_cast<cudaStream_t>(stream), 2000000000ull, nullptr);
 }

@@ -76,4 +76,8 @@ inline int launch_pairs_emulated(const void* fn, int grid, int world, size_t sme
 }
 
 }  // namespace gemm
+namespace gemm2 {
+// gemm2.cu: C = A * Bt^T on CTA pairs; grid <= 0: one CTA per SM
+int launch_gemm_pair(const tccl_gemm_args* g, int grid, cudaStream_t stream, uint64_t timeout_ns, uint64_t* trace);
+}  // namespace gemm2
 }  // namespace tccl

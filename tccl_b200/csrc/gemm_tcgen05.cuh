@@ -349,5 +349,8 @@ __device__ __forceinline__ Vec16 pack8_bf16(const uint32_t* r) {
   return v;
 }
 
+// silu(g) * u
+__device__ __forceinline__ float swiglu(float g, float u) { return g / (1.f + __expf(-g)) * u; }
+
 }  // namespace gemm
 }  // namespace tccl

@@ -48,6 +48,11 @@ __device__ __forceinline__ uint32_t cluster_ctarank() {
 __device__ __forceinline__ void cluster_sync() {
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
+// the pair leaves together: orders nothing but the lifetime of shared and tensor memory, so no release (a release
+// here waited ~1 us for the epilogue's global stores to be acknowledged)
+__device__ __forceinline__ void cluster_sync_relaxed() {
+  asm volatile("barrier.cluster.arrive.relaxed.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
+}
 // address of the same shared-memory location in CTA `cta` of the cluster
 __device__ __forceinline__ uint32_t mapa(uint32_t smem_addr, uint32_t cta) {
   uint32_t r;
@@ -111,6 +116,103 @@ struct Smem2 {
     epi[1] = epi[0] + kEpiChunkBytes;
   }
 };
+
+// Order of `tm` x `tn` pair tiles for tiles that a persistent grid takes in steps of its size: groups of `g` tile
+// rows, inside a group column by column.  The tiles running at one time then span g rows and pairs / g columns, so
+// what the grid reads per k-block is about (g + pairs / g) tiles of 256 rows instead of (pairs / tn + tn), and the
+// A rows of a group stay in L2 from one wave to the next while Bt streams past once per group.  Row-major order read
+// all of a wide Bt once per tile row: 16 x 235 MB for [4096, 4096] x [28672, 4096]^T, which bound that product
+// (883 us, 1.09 PFLOP/s; grouped: see raster_group).
+struct Raster {
+  int tn, g, tm;
+  __device__ __forceinline__ void at(int t, int& m, int& n) const {
+    const int per = g * tn, grp = t / per, r = t - grp * per;
+    const int m0 = grp * g, rows = min(g, tm - m0);
+    n = r / rows;
+    m = m0 + (r - n * rows);
+  }
+};
+// Tile rows per group: as many as keep the group's A rows (512 K bytes each) in about a third of L2, but at least
+// 8, near the square root of the 74 pairs, where a wave reads least.
+inline int raster_group(int tm, int k) {
+  const long long fit = (48ll << 20) / (512ll * k);
+  const int want = (int)(fit < 8 ? 8 : (fit > 24 ? 24 : fit));
+  const int groups = (tm + want - 1) / want;
+  return (tm + groups - 1) / groups;  // groups of equal height
+}
+
+// Tile order of a persistent grid of `pairs` CTA pairs over `total` 256 x 256 tiles: the
+// whole waves first (unit = pair + i * pairs), then the tiles of the last, partial wave cut
+// into left and right halves, so that the tail costs every pair at most half a tile more
+// than the pairs that are done.
+struct TailSplitSchedule {
+  int total, pairs, nfull, rem;
+  __host__ __device__ void init(int total_, int pairs_) {
+    total = total_;
+    pairs = pairs_;
+    nfull = (total / pairs) * pairs;
+    rem = total - nfull;
+  }
+  __device__ __forceinline__ bool unit(int pair, int i, int& tile, int& half) const {
+    const int u = pair + i * pairs;
+    if (u < nfull) {
+      tile = u;
+      half = 0;
+      return true;
+    }
+    const int h = u - nfull;
+    if (h >= 2 * rem) return false;
+    tile = nfull + (h >> 1);
+    half = 1 + (h & 1);
+    return true;
+  }
+};
+
+// Epilogue piece: this warp's 32 rows x 64 columns of fp32 (pairs of registers r[2 i], r[2 i + 1] -> one bf16x2), one
+// row per lane, to global memory through the warp's own 4 KB of shared memory.  Stores straight from the registers
+// put 16 bytes into each of 32 rows per instruction (one L1 pass per row: 2.5 us for a 128 x 256 tile); after the
+// exchange 8 lanes cover 128 contiguous bytes of one row (4 passes).  `buf`: 16-byte vector v of row r sits at
+// position v ^ (r & 7): no bank conflicts either way.
+__device__ __forceinline__ void stage_put(uint8_t* buf, int lane, int v, const Vec16& x) {
+  st_shared_v4(buf + lane * 128 + ((v ^ (lane & 7)) << 4), x);
+}
+__device__ __forceinline__ Vec16 ld_shared_v4(const void* p) {
+  Vec16 v;
+  asm volatile("ld.shared.v4.b32 {%0,%1,%2,%3}, [%4];"
+               : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(smem_u32(p)) : "memory");
+  return v;
+}
+// `dst`: row 0, column 0 of the piece; rows / columns beyond `nrows` / `ncols` are not stored (ncols % 8 == 0)
+__device__ __forceinline__ void stage_flush(const uint8_t* buf, int lane, __nv_bfloat16* dst, size_t ld, int nrows,
+                                            int ncols) {
+  __syncwarp();
+  const int v = lane & 7;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const int row = i * 4 + (lane >> 3);
+    const Vec16 x = ld_shared_v4(buf + row * 128 + ((v ^ (row & 7)) << 4));
+    if (row < nrows && v * 8 < ncols) st_local(dst + (size_t)row * ld + v * 8, x);
+  }
+  __syncwarp();
+}
+// `ncols` (64, 128, ...) accumulator columns at `taddr` -> bf16 at C's rows from `row0` on, columns from `col` on
+__device__ __forceinline__ void store_rows(uint8_t* buf, __nv_bfloat16* C, size_t ldc, int row0, int M, int col, int N,
+                                           int ncols, uint32_t taddr, int lane) {
+  __nv_bfloat16* dst = C + (size_t)row0 * ldc + col;
+#pragma unroll 1
+  for (int c = 0; c < ncols; c += 64) {
+    uint32_t r[32], q[32];
+    tmem_ld_32x32(taddr + c, r);
+    tmem_ld_32x32(taddr + c + 32, q);
+    tmem_ld_wait();
+#pragma unroll
+    for (int v = 0; v < 4; ++v) {
+      stage_put(buf, lane, v, pack8_bf16(r + v * 8));
+      stage_put(buf, lane, v + 4, pack8_bf16(q + v * 8));
+    }
+    stage_flush(buf, lane, dst + c, ldc, M - row0, N - col - c);
+  }
+}
 
 // `half`: 0 = the full 256 columns of n tile nt, 1 / 2 = its left / right 128 columns
 // Hooks (Policy):
@@ -262,7 +364,7 @@ __device__ void run_mainloop2(const Shape shp, Policy& pol, const tccl_comm* com
   // unless a wait failed, in which case the deadline (seconds) has long outlasted any copy.
   tc_fence_before();
   __syncthreads();
-  cluster_sync();
+  cluster_sync_relaxed();
   if (warp == 2) {
     tc_fence_after();
     tmem_dealloc2(tmem_base, kTmemCols);
