@@ -242,6 +242,7 @@ struct AgGemmPairPolicy {
   }
 
   __device__ __forceinline__ bool before_load(int mt, int, const Abort& ab) const {
+    if (c->world == 1) return true;  // (also for the row tile that hangs over the end)
     const int src = mt / p->tiles_m_per_rank;
     if (src == c->rank) return true;
     const int rt = mt - src * p->tiles_m_per_rank;
@@ -252,7 +253,7 @@ struct AgGemmPairPolicy {
     return ok;
   }
   __device__ __forceinline__ void a_tile(int mt, const CUtensorMap*& map, int& y) const {
-    const int src = mt / p->tiles_m_per_rank;
+    const int src = c->world == 1 ? 0 : mt / p->tiles_m_per_rank;
     if (src == c->rank) {
       map = &p->map_a_shard;
       y = (mt - src * p->tiles_m_per_rank) * 128;
@@ -266,27 +267,7 @@ struct AgGemmPairPolicy {
     const int row0 = mt * 128 + quad * 32;
     uint8_t* buf = sm.epi[0] + quad * 4096;
     if (p->swiglu) {
-      // every 256-wide tile holds 128 gate columns followed by the 128 matching up columns; a half
-      // tile's accumulator holds 64 of each (see b_tile)
-      const int hw = ncols / 2, col = nt * (BN2 / 2) + col_lo / 2;
-#pragma unroll 1
-      for (int c = 0; c < hw; c += 64) {
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          uint32_t g[32], u[32];
-          tmem_ld_32x32(taddr + c + h * 32, g);
-          tmem_ld_32x32(taddr + hw + c + h * 32, u);
-          tmem_ld_wait();
-#pragma unroll
-          for (int v = 0; v < 4; ++v) {
-            uint32_t o[8];
-#pragma unroll
-            for (int e = 0; e < 8; ++e) o[e] = __float_as_uint(swiglu(__uint_as_float(g[v * 8 + e]), __uint_as_float(u[v * 8 + e])));
-            stage_put(buf, lane, h * 4 + v, pack8_bf16(o));
-          }
-        }
-        stage_flush(buf, lane, p->out + (size_t)row0 * p->ldo + col + c, p->ldo, p->shp.M - row0, p->shp.N / 2 - col - c);
-      }
+      store_rows_swiglu(buf, p->out, p->ldo, row0, p->shp.M, nt * (BN2 / 2) + col_lo / 2, p->shp.N / 2, ncols / 2, taddr, lane);
       return true;
     }
     // a half tile's 128 columns sit at the start of the accumulator
@@ -346,7 +327,8 @@ static int fill_params(AgGemmPairParams* p, const tccl_ag_gemm_args* g, int worl
   if (g->m <= 0 || g->n <= 0 || g->k <= 0) return -TCCL_EINVAL;
   if ((g->lda_shard % 8) || (g->lda_full % 8) || (g->ldb % 8) || (g->ldo % 8) || (g->k % 8) || (g->n % 8))
     return -TCCL_EALIGN;
-  if (g->m % (world * 256)) return -TCCL_ESIZE;  // whole 256-row pair tiles per rank
+  // whole 256-row pair tiles per rank (one rank: the last pair tile may hang over the end)
+  if (g->m % (world == 1 ? 128 : world * 256)) return -TCCL_ESIZE;
   if (((uintptr_t)g->a_shard | (uintptr_t)g->bt | (uintptr_t)g->out | (uintptr_t)g->a_full[rank] | half_bytes) & 15)
     return -TCCL_EALIGN;
   const int rows = g->m / world;
@@ -375,8 +357,8 @@ static int fill_params(AgGemmPairParams* p, const tccl_ag_gemm_args* g, int worl
   p->ldo = g->ldo;
   p->tiles_n = (g->n + BN2 - 1) / BN2;
   p->tiles_m_per_rank = rows / 128;
-  p->raster = Raster{p->tiles_n, raster_group(rows / 256, g->k), rows / 256};
-  p->tail.init(rows / 256 * p->tiles_n, pairs);
+  p->raster = Raster{p->tiles_n, raster_group((rows + 255) / 256, g->k), (rows + 255) / 256};
+  p->tail.init((rows + 255) / 256 * p->tiles_n, pairs);
   p->swiglu = g->swiglu;
   p->batches = g->comm_ctas > 0 ? g->comm_ctas : 2;
   p->movers_only = (g->lsu_movers & 2) != 0;

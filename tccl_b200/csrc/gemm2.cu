@@ -10,7 +10,8 @@ namespace gemm2 {
 struct PlainPolicy2 {
   const CUtensorMap *map_a, *map_b128, *map_b64;
   __nv_bfloat16* C;
-  int M, N, ldc;
+  int M, N, ldc;  // N: rows of Bt
+  int swiglu;
   Raster raster;
   TailSplitSchedule sched;
   __device__ __forceinline__ bool tile(int i, int& mt, int& nt, int& half) const {
@@ -22,7 +23,8 @@ struct PlainPolicy2 {
   }
   __device__ __forceinline__ void b_tile(int nt, int half, int cta, const CUtensorMap*& map, int& y) const {
     map = half ? map_b64 : map_b128;
-    y = b_rows_default(nt, half, cta);
+    // gate | up packing: a half tile is 64 gate columns (CTA 0) and the 64 matching up columns (CTA 1)
+    y = (swiglu && half) ? nt * BN2 + cta * 128 + (half == 2 ? 64 : 0) : b_rows_default(nt, half, cta);
   }
   __device__ __forceinline__ bool before_load(int, int, const Abort&) const { return true; }
   __device__ __forceinline__ void a_tile(int mt, const CUtensorMap*& map, int& y) const {
@@ -34,6 +36,11 @@ struct PlainPolicy2 {
   __device__ __forceinline__ void epilogue_begin(int, int, const Abort&) const {}
   __device__ __forceinline__ bool epilogue(int mt, int nt, int col0, int ncols, uint32_t taddr, int quad, int lane,
                                            const Abort&, const Smem2& sm) const {
+    if (swiglu) {
+      store_rows_swiglu(sm.epi[0] + quad * 4096, C, ldc, mt * 128 + quad * 32, M, nt * (BN2 / 2) + col0 / 2, N / 2,
+                        ncols / 2, taddr, lane);
+      return true;
+    }
     store_rows(sm.epi[0] + quad * 4096, C, ldc, mt * 128 + quad * 32, M, nt * BN2 + col0, N, ncols, taddr, lane);
     return true;
   }
@@ -55,6 +62,8 @@ int launch_gemm_pair(const tccl_gemm_args* g, int grid, cudaStream_t stream, uin
   if (!g || g->m <= 0 || g->n <= 0 || g->k <= 0) return -TCCL_EINVAL;
   if ((g->lda % 8) || (g->ldb % 8) || (g->ldc % 8) || (g->n % 8) || (g->k % 8)) return -TCCL_EALIGN;
   if (((uintptr_t)g->a | (uintptr_t)g->bt | (uintptr_t)g->c) & 15) return -TCCL_EALIGN;
+  if (g->swiglu && (g->n % BN2)) return -TCCL_ESIZE;  // whole gate|up tiles only
+  if (grid <= 0 && g->m <= kSkinnyMaxRows && !trace) return launch_gemm_skinny(g, stream);
   CUtensorMap ma, mb128, mb64;
   int rc = make_tmap_bf16_kmajor(&ma, g->a, g->m, g->k, g->lda, 128);  // each CTA loads 128 rows of A ...
   if (rc) return rc;
@@ -67,6 +76,7 @@ int launch_gemm_pair(const tccl_gemm_args* g, int grid, cudaStream_t stream, uin
   pol.M = g->m;
   pol.N = g->n;
   pol.ldc = g->ldc;
+  pol.swiglu = g->swiglu;
   const int tm = (g->m + 255) / 256, tn = (g->n + BN2 - 1) / BN2, total = tm * tn;
   pol.raster = Raster{tn, raster_group(tm, g->k), tm};
   if (grid <= 0) grid = tccl_num_sms();

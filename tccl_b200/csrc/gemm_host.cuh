@@ -77,7 +77,10 @@ inline int launch_pairs_emulated(const void* fn, int grid, int world, size_t sme
 
 }  // namespace gemm
 namespace gemm2 {
-// gemm2.cu: C = A * Bt^T on CTA pairs; grid <= 0: one CTA per SM
+// Products of up to this many rows go to the kernel for few rows (gemm_skinny.cu).
+constexpr int kSkinnyMaxRows = 128;
+int launch_gemm_skinny(const tccl_gemm_args* g, cudaStream_t stream);
+// gemm2.cu: C = A * Bt^T on CTA pairs; grid <= 0: one CTA per SM, and the kernel that suits the shape
 int launch_gemm_pair(const tccl_gemm_args* g, int grid, cudaStream_t stream, uint64_t timeout_ns, uint64_t* trace);
 }  // namespace gemm2
 }  // namespace tccl

@@ -324,12 +324,10 @@ extern "C" int tccl_gemm_reduce_scatter_pair(const tccl_comm* comm, const tccl_g
   if (comm->world == 1) {
     // One rank: the partial is the result.  The plain product stores it once; through the staging area it took
     // two more passes over [m, n] and the flag traffic (4096 x 4096 x 14336: 403 us).
-    GemmRsPairParams check;
-    const int rc = fill_params(&check, args, 1, l->n_emu ? stage_bytes : comm->stage_bytes, 0);
-    if (rc) return rc;
+    if ((args->n % BN2) || (args->m % 128)) return -TCCL_ESIZE;
     const tccl_gemm_args g{args->a, args->bt, args->out, comm->local + TCCL_LOCAL_STATUS, args->m, args->n, args->k,
-                           args->lda, args->ldb, args->ldo};
-    return launch_gemm_pair(&g, l->grid, s, comm->timeout_ns, reinterpret_cast<uint64_t*>(args->trace));
+                           args->lda, args->ldb, args->ldo, 0};
+    return launch_gemm_pair(&g, args->trace ? l->grid : 0, s, comm->timeout_ns, reinterpret_cast<uint64_t*>(args->trace));
   }
   static bool attr_set = false;
   if (!attr_set) {

@@ -214,6 +214,32 @@ __device__ __forceinline__ void store_rows(uint8_t* buf, __nv_bfloat16* C, size_
   }
 }
 
+// The same with the SwiGLU product of two column blocks of one tile: gate columns at `taddr`, the matching up columns
+// `ncols` further on (every 256-wide tile of a packed Bt holds 128 gate columns followed by the 128 matching up columns,
+// a half tile 64 of each).  `N`, `col`: of the [M, N / 2] result.
+__device__ __forceinline__ void store_rows_swiglu(uint8_t* buf, __nv_bfloat16* C, size_t ldc, int row0, int M, int col,
+                                                  int N, int ncols, uint32_t taddr, int lane) {
+#pragma unroll 1
+  for (int c = 0; c < ncols; c += 64) {
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      uint32_t g[32], u[32];
+      tmem_ld_32x32(taddr + c + h * 32, g);
+      tmem_ld_32x32(taddr + ncols + c + h * 32, u);
+      tmem_ld_wait();
+#pragma unroll
+      for (int v = 0; v < 4; ++v) {
+        uint32_t o[8];
+#pragma unroll
+        for (int e = 0; e < 8; ++e)
+          o[e] = __float_as_uint(swiglu(__uint_as_float(g[v * 8 + e]), __uint_as_float(u[v * 8 + e])));
+        stage_put(buf, lane, h * 4 + v, pack8_bf16(o));
+      }
+    }
+    stage_flush(buf, lane, C + (size_t)row0 * ldc + col + c, ldc, M - row0, N - col - c);
+  }
+}
+
 // `half`: 0 = the full 256 columns of n tile nt, 1 / 2 = its left / right 128 columns
 // Hooks (Policy):
 //   tile(i, mt, nt, half)                  -> false when the PAIR is out of tiles; mt is even

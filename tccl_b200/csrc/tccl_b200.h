@@ -254,11 +254,14 @@ typedef struct tccl_gemm_args {
   void* status;    /* optional: TCCL_ST_WORDS uint32 words for a timeout report, or NULL */
   int32_t m, n, k;
   int32_t lda, ldb, ldc;
+  int32_t swiglu;  /* tccl_gemm_bf16_pair only.  1: every 256-row block of bt is 128 gate rows then the 128 matching up
+                      rows (n % 256 == 0); c is [m, n / 2] = silu(gate) * up */
 } tccl_gemm_args;
 /* c = a * bt^T on this GPU; grid <= 0 picks one CTA per SM */
 int tccl_gemm_bf16(const tccl_gemm_args*, int grid, void* stream);
 /* same product on pairs of CTAs (tcgen05.mma.cta_group::2): 256 x 256 tiles, each CTA loads its own
- * 128 rows of a and its own half of bt; the last partial wave is cut into 256 x 128 half tiles */
+ * 128 rows of a and its own half of bt; the last partial wave is cut into 256 x 128 half tiles.
+ * With grid <= 0 products of few rows take a kernel of their own. */
 int tccl_gemm_bf16_pair(const tccl_gemm_args*, int grid, void* stream);
 
 /* ---- fused GEMM -> reduce-scatter (rows scattered over the ranks) ---------- */

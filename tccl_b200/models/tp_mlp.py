@@ -23,7 +23,7 @@ from typing import Optional
 import torch
 
 from ..ops.fused import all_gather_gemm, all_reduce_bias_residual_rmsnorm, gemm_reduce_scatter, pack_gate_up
-from ..ops.gemm import gemm_bf16
+from ..ops.gemm import gemm_bf16, gemm_swiglu_bf16
 from ..parallel.world import WorldBase
 
 
@@ -62,9 +62,7 @@ class TensorParallelMLP:
     # -- replicated in, replicated out: local GEMMs + one fused all-reduce/norm kernel
     def forward_allreduce(self, x: torch.Tensor, residual: Optional[torch.Tensor] = None, eps: float = 1e-5):
         T = x.shape[0]
-        gu = gemm_bf16(x, self.gate_up_packed)                     # [T, 2 * inter_local], packed gate|up per 256
-        gu = gu.view(T, -1, 2, 128)
-        act = (torch.nn.functional.silu(gu[:, :, 0].float()) * gu[:, :, 1].float()).to(torch.bfloat16).reshape(T, -1)
+        act = gemm_swiglu_bf16(x, self.gate_up_packed)             # [T, inter_local]
         key = ("partial", T)
         buf = self.__dict__.setdefault("_bufs", {})
         if key not in buf:

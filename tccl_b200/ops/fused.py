@@ -138,11 +138,12 @@ def _plan_gemm_rs(w, As, Bs, Os, variant) -> FusedPlan:
     if variant not in ("auto", "pair", "single"):
         raise ValueError("variant must be 'auto', 'pair' or 'single'")
     pair_ok = M % (W * 256) == 0 and lib.tccl_gemm_rs_pair_stage_bytes(M, N, W) <= stage_bytes
+    local = W == 1 and variant != "single"  # one rank: the plain product, no staging area, any row count
     if variant == "pair" and not pair_ok:
         raise ValueError(f"the pair kernel needs M % {W * 256} == 0 and "
                          f"{lib.tccl_gemm_rs_pair_stage_bytes(M, N, W) >> 20} MiB of staging area")
-    pair = pair_ok and variant != "single"
-    need = lib.tccl_gemm_rs_pair_stage_bytes(M, N, W) if pair else lib.tccl_gemm_rs_stage_bytes(M, N, W)
+    pair = (pair_ok or local) and variant != "single"
+    need = 0 if local else lib.tccl_gemm_rs_pair_stage_bytes(M, N, W) if pair else lib.tccl_gemm_rs_stage_bytes(M, N, W)
     if need > stage_bytes:
         raise ValueError(f"staging area too small: need {need >> 20} MiB, have {w.config.stage_mb} MiB "
                          "(raise TCCL_STAGE_MB)")
@@ -289,7 +290,8 @@ def _plan_ag_gemm(w, As, Bs, a_full, Os, comm_ctas, swiglu, lsu_movers, variant)
     pair_ok = rows % 256 == 0
     if variant == "pair" and not pair_ok:
         raise ValueError("the pair kernel needs (M / W) % 256 == 0")
-    pair = pair_ok and variant != "single"
+    # one rank: the last pair tile may hang over the end of the rows
+    pair = (pair_ok or (W == 1 and variant == "auto")) and variant != "single"
     half_bytes = 0
     views = None
     if a_full is None:
