@@ -277,6 +277,7 @@ struct AgGemmPairPolicy {
 };
 
 __device__ __forceinline__ void ag_gemm_pair_body(const tccl_comm& c, const AgGemmPairParams& p, int bid, int nb) {
+  grid_dependency_wait();
   const uint32_t epoch = c.local[TCCL_LOCAL_TILE_EPOCH] + 1u;
   const int parity = p.half_bytes ? (int)(c.local[TCCL_LOCAL_AG_SEQ] & 1u) : 0;
   if (!p.half_bytes) {
@@ -397,8 +398,7 @@ extern "C" int tccl_allgather_gemm_pair(const tccl_comm* comm, const tccl_ag_gem
     AgGemmPairParams p;
     int rc = fill_params(&p, args, comm->world, comm->rank, l->grid / 2, half_bytes);
     if (rc) return rc;
-    ag_gemm_pair_kernel<<<l->grid, kThreads, kSmem2, s>>>(*comm, p);
-    return (int)cudaGetLastError();
+    return tccl::launch_dependent(ag_gemm_pair_kernel, dim3(l->grid), kThreads, kSmem2, s, 0, *comm, p);
   }
   const int W = l->n_emu;
   if (W < 1 || W > TCCL_MAX_WORLD) return -TCCL_EINVAL;

@@ -303,12 +303,43 @@ struct Entry {
   }
 };
 
+// ------------------------------------------------- programmatic dependent launch
+// A kernel launched with `programmatic` set may be resident before the previous kernel of its stream has
+// finished: its launch and its set-up overlap the predecessor's last CTAs (1.4 - 1.7 us per kernel of a chain of
+// small ones).  grid_dependency_wait returns when every earlier kernel of the stream is complete and its writes
+// are visible; nothing that another kernel may read or write is touched before it.  The successor is let in
+// after that, so at most one kernel waits behind the running one.
+__device__ __forceinline__ void grid_dependency_wait() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+// launch of a kernel that calls grid_dependency_wait; `cluster` CTAs per cluster along x (0: none or compile-time)
+template <class... Params, class... Args>
+inline int launch_dependent(void (*kernel)(Params...), dim3 grid, int block, size_t smem, cudaStream_t stream, int cluster,
+                            const Args&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = cluster;
+  attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = cluster ? 2 : 1;
+  return (int)cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
 // ---------------------------------------------------------- kernel scaffolding
 // Every collective is a struct `Op` with `using Args = ...` and
 // `static __device__ void run(const tccl_comm&, const Args&, int bid, int nblocks)`.
 template <class Op>
 __global__ void __launch_bounds__(Op::kMaxThreads, Op::kMinBlocks)
 kernel_real(const __grid_constant__ tccl_comm comm, const __grid_constant__ typename Op::Args args) {
+  grid_dependency_wait();
   Op::run(comm, args, blockIdx.x, gridDim.x);
 }
 // Emulated ranks: the structs of all ranks travel as one kernel parameter (under the 32 KB that sm_70 and
@@ -332,8 +363,7 @@ inline int launch_op(const tccl_comm* comm, const typename Op::Args* args, const
   if (l->n_emu == 0) {
     if (smem > 48 * 1024)
       cudaFuncSetAttribute(kernel_real<Op>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    kernel_real<Op><<<l->grid, l->block, smem, s>>>(*comm, *args);
-    return (int)cudaGetLastError();
+    return launch_dependent(kernel_real<Op>, dim3(l->grid), l->block, smem, s, 0, *comm, *args);
   }
   if (l->n_emu < 0 || l->n_emu > TCCL_MAX_WORLD) return -TCCL_EINVAL;
   EmuParams<typename Op::Args> p;

@@ -63,9 +63,10 @@ int launch_gemm_pair(const tccl_gemm_args* g, int grid, cudaStream_t stream, uin
   if ((g->lda % 8) || (g->ldb % 8) || (g->ldc % 8) || (g->n % 8) || (g->k % 8)) return -TCCL_EALIGN;
   if (((uintptr_t)g->a | (uintptr_t)g->bt | (uintptr_t)g->c) & 15) return -TCCL_EALIGN;
   if (g->swiglu && (g->n % BN2)) return -TCCL_ESIZE;  // whole gate|up tiles only
-  if (grid <= 0 && g->m <= kSkinnyMaxRows && !trace) return launch_gemm_skinny(g, stream);
+  int rc = 0;
+  if (grid <= 0 && !trace && launch_gemm_skinny(g, stream, &rc)) return rc;
   CUtensorMap ma, mb128, mb64;
-  int rc = make_tmap_bf16_kmajor(&ma, g->a, g->m, g->k, g->lda, 128);  // each CTA loads 128 rows of A ...
+  rc = make_tmap_bf16_kmajor(&ma, g->a, g->m, g->k, g->lda, 128);  // each CTA loads 128 rows of A ...
   if (rc) return rc;
   rc = make_tmap_bf16_kmajor(&mb128, g->bt, g->n, g->k, g->ldb, 128);  // ... and 128 rows of Bt (64 for a half tile)
   if (rc) return rc;
@@ -92,9 +93,8 @@ int launch_gemm_pair(const tccl_gemm_args* g, int grid, cudaStream_t stream, uin
     attr_set = true;
   }
   Shape shp{g->m, g->n, g->k};
-  gemm_pair_kernel<<<grid, kThreads, kSmem2, stream>>>(ma, mb128, mb64, shp, pol, reinterpret_cast<uint32_t*>(g->status),
-                                                       timeout_ns, trace);
-  return (int)cudaGetLastError();
+  return launch_dependent(gemm_pair_kernel, dim3(grid), kThreads, kSmem2, stream, 0, ma, mb128, mb64, shp, pol,
+                          reinterpret_cast<uint32_t*>(g->status), timeout_ns, trace);
 }
 
 }  // namespace gemm2

@@ -215,6 +215,7 @@ struct GemmRsPairPolicy {
 
 __device__ __forceinline__ void gemm_rs_pair_body(const tccl_comm& c, const GemmRsPairParams& p, int bid, int nb) {
   __shared__ int s_unit;
+  grid_dependency_wait();
   const uint64_t deadline = globaltimer() + c.timeout_ns;
   GemmRsPairPolicy pol;
   pol.c = &c;
@@ -341,8 +342,7 @@ extern "C" int tccl_gemm_reduce_scatter_pair(const tccl_comm* comm, const tccl_g
     GemmRsPairParams p;
     int rc = fill_params(&p, args, comm->world, comm->stage_bytes, sync_entry);
     if (rc) return rc;
-    gemm_rs_pair_kernel<<<l->grid, kThreads, kSmem2, s>>>(*comm, p);
-    return (int)cudaGetLastError();
+    return tccl::launch_dependent(gemm_rs_pair_kernel, dim3(l->grid), kThreads, kSmem2, s, 0, *comm, p);
   }
   const int W = l->n_emu;
   if (W < 1 || W > TCCL_MAX_WORLD) return -TCCL_EINVAL;

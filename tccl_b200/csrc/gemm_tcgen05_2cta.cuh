@@ -294,6 +294,7 @@ __device__ void run_mainloop2(const Shape shp, Policy& pol, const tccl_comm* com
   cluster_sync();  // both CTAs' barriers are initialised before anyone signals across
   tc_fence_after();
   const uint32_t tmem_base = *sm.tmem_base;
+  grid_dependency_wait();
   Abort ab{sm.abort_flag, comm, comm ? comm->local + TCCL_LOCAL_STATUS : nullptr, globaltimer() + timeout_ns};
 
   if (warp == 0) {
