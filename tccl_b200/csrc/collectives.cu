@@ -380,8 +380,30 @@ struct AllReduceTwoShotNvls {
 };
 
 // ------------------------------------------------------------ all-gather, pull
-// out[p][i] = in_p[i]; the peer order starts at the own rank and every CTA
-// walks it from a different offset so that the W-1 streams spread over peers.
+// out[p][i] = in_p[i].  The slabs of all W shards are dealt to the CTAs in one sequence, shard fastest and starting at
+// the own rank: neighbouring CTAs read different peers, and a small message is one round of loads (shard after shard,
+// every CTA waited for W rounds in turn).
+//
+// A shard whose size is no multiple of 16 bytes puts the slots of ranks >= 1 off the 16-byte grid.  Both sides are
+// still moved as whole aligned vectors: the 16 bytes that belong at a destination vector are the end of source vector
+// j and the start of j + 1, which the next lane has loaded, so a shuffle and a funnel shift by a per-slot constant put
+// them together (the last lane of a warp loads one vector more: 32 bytes for every 512).  One element per thread and
+// iteration, as before, left one load in flight per thread: 4 emulated ranks x 1000003 fp32 (80 MB of traffic) took
+// 76 us, this way 30 us.
+
+// Bytes `head` .. `head` + 15 of lo | hi (head: 0 .. 15, even).
+__device__ __forceinline__ Vec16 realign(const Vec16& lo, const Vec16& hi, uint32_t head) {
+  const uint32_t w[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
+  uint32_t a[6], b[5], r[4];
+#pragma unroll
+  for (int i = 0; i < 6; ++i) a[i] = head & 8 ? w[i + 2] : w[i];
+#pragma unroll
+  for (int i = 0; i < 5; ++i) b[i] = head & 4 ? a[i + 1] : a[i];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) r[i] = __funnelshift_r(b[i], b[i + 1], (head & 3) * 8);
+  return Vec16{r[0], r[1], r[2], r[3]};
+}
+
 template <typename T, int W>
 struct AllGatherPullP2P {
   using Args = tccl_coll_args;
@@ -390,36 +412,74 @@ struct AllGatherPullP2P {
   static __device__ void run(const tccl_comm& c, const Args& a, int bid, int nb) {
     Entry sync(c, a.flags, bid);
     const int world = WorldOf<W>::get(c);
-    constexpr int VPT = VecOf<T>::n;
-    const uint64_t nvec = a.numel / VPT;
-    const uint64_t bs = blockDim.x;
-    const uint64_t nthr = (uint64_t)nb * blockDim.x;
-    const uint64_t tid = (uint64_t)bid * blockDim.x + threadIdx.x;
-    if ((a.numel * sizeof(T)) & 15) {
-      // shard size not a multiple of 16 bytes: the output slots of ranks >= 1 are
-      // not vector aligned, so copy element by element
-      for (int k = 0; k < world; ++k) {
-        const int p = (c.rank + k + bid) % world;
-        const volatile T* src = reinterpret_cast<const volatile T*>(a.in[p]);
-        T* dst = reinterpret_cast<T*>(a.out) + (uint64_t)p * a.numel;
-        for (uint64_t e = tid; e < a.numel; e += nthr) dst[e] = src[e];
+    const uint64_t bytes = a.numel * sizeof(T), nvec = bytes / 16;  // whole vectors of a shard
+    const uint32_t bs = blockDim.x;
+    const uint64_t slabs = (nvec + bs * U - 1) / (bs * U) * world;
+    auto shard = [&](uint64_t it) {
+      const int p = c.rank + (int)(it % world);
+      return p >= world ? p - world : p;
+    };
+    if (bytes & 15) {
+      // vectors 0 .. body - 1 of the destination grid need source vectors 0 .. body; the shuffles want whole warps
+      const uint64_t body = (nvec < 2 || (bs & 31)) ? 0 : nvec - 1;
+      const int lane = threadIdx.x & 31;
+      Vec16 v[U], x[U];
+      auto load = [&](uint64_t it) {
+        const void* src = a.in[shard(it)];
+        const uint64_t i0 = it / world * bs * U + threadIdx.x;
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          const uint64_t i = i0 + u * bs;
+          if (i < nvec && TCCL_VIN(c, a, i)) v[u] = ld_peer(vptr<T>(src, i));
+          if (lane == 31 && i + 1 < nvec && TCCL_VIN(c, a, i + 1)) x[u] = ld_peer(vptr<T>(src, i + 1));
+        }
+      };
+      uint64_t it = bid;
+      if (body && it < slabs) load(it);
+      while (body && it < slabs) {
+        const uint64_t slot = (uint64_t)shard(it) * bytes;
+        const uint32_t head = (uint32_t)(0 - slot) & 15u;  // bytes of the slot before its first aligned vector
+        const uint64_t i0 = it / world * bs * U + threadIdx.x;
+        Vec16 r[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          Vec16 n{__shfl_down_sync(0xffffffffu, v[u].x, 1), __shfl_down_sync(0xffffffffu, v[u].y, 1),
+                  __shfl_down_sync(0xffffffffu, v[u].z, 1), __shfl_down_sync(0xffffffffu, v[u].w, 1)};
+          if (lane == 31) n = x[u];
+          r[u] = realign(v[u], n, head);
+        }
+        it += nb;
+        if (it < slabs) load(it);  // the next slab is on its way while this one is stored
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          const uint64_t i = i0 + u * bs, off = slot + head + i * 16;
+          if (i < body && TCCL_IN_BOUNDS(c, off, 16, a.out_bytes, TCCL_W_INDEX_OUT))
+            st_local(reinterpret_cast<char*>(a.out) + off, r[u]);
+        }
+      }
+      // what lies before a slot's first aligned vector and after its last: at most 31 bytes of each shard
+      const uint64_t bodye = body * 16 / sizeof(T), rest = a.numel - bodye;
+      for (uint64_t j = (uint64_t)bid * bs + threadIdx.x; j < rest * world; j += (uint64_t)nb * bs) {
+        const uint64_t p = j / rest, e0 = j - p * rest;
+        const uint64_t heade = ((uint32_t)(0 - p * bytes) & 15u) / sizeof(T);
+        const uint64_t e = e0 < heade ? e0 : e0 + bodye;
+        reinterpret_cast<T*>(a.out)[p * a.numel + e] = reinterpret_cast<const volatile T*>(a.in[p])[e];
       }
       sync.exit(c, a.flags, bid);
       return;
     }
-    for (int k = 0; k < world; ++k) {
-      const int p = (c.rank + k + bid) % world;
+    for (uint64_t it = bid; it < slabs; it += nb) {
+      const int p = shard(it);
       const void* src = a.in[p];
-      char* dst = reinterpret_cast<char*>(a.out) + (uint64_t)p * a.numel * sizeof(T);
-      TCCL_FOR_SLABS(U, nvec, bid, nb, i0) {
-        Vec16 v[U];
+      char* dst = reinterpret_cast<char*>(a.out) + (uint64_t)p * bytes;
+      const uint64_t i0 = it / world * bs * U + threadIdx.x;
+      Vec16 v[U];
 #pragma unroll
-        for (int u = 0; u < U; ++u)
-          if (i0 + u * bs < nvec && TCCL_VIN(c, a, i0 + u * bs)) v[u] = ld_peer(vptr<T>(src, i0 + u * bs));
+      for (int u = 0; u < U; ++u)
+        if (i0 + u * bs < nvec && TCCL_VIN(c, a, i0 + u * bs)) v[u] = ld_peer(vptr<T>(src, i0 + u * bs));
 #pragma unroll
-        for (int u = 0; u < U; ++u)
-          if (i0 + u * bs < nvec && TCCL_VOUT(c, a, (uint64_t)p * nvec + i0 + u * bs)) st_local(dst + (i0 + u * bs) * 16, v[u]);
-      }
+      for (int u = 0; u < U; ++u)
+        if (i0 + u * bs < nvec && TCCL_VOUT(c, a, (uint64_t)p * nvec + i0 + u * bs)) st_local(dst + (i0 + u * bs) * 16, v[u]);
     }
     sync.exit(c, a.flags, bid);
   }

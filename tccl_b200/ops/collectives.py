@@ -430,7 +430,9 @@ def _plan_all_gather(w, x, out, algo, sync_exit) -> Plan:
     block = w.config.block
     if algo == "pull":
         args = {r: _copy_args(base) for r in w.local_ranks}
-        go = w.prepare("tccl_allgather_pull_p2p", args, grid_for(w, nvec, block, 4), block, dt)
+        # slabs of block x 8 vectors, per shard
+        grid = grid_for(w, W * -(-nvec // (block * 8)), 1, 1)
+        go = w.prepare("tccl_allgather_pull_p2p", args, grid, block, dt)
         if out is not None:
             for r, a in args.items():
                 o = w.local(out, r)

@@ -225,6 +225,30 @@ def test_all_gather_pull(emu_worlds, W, dtype, n):
         assert torch.equal(out[r], ref)
 
 
+@pytest.mark.parametrize("W,block", [(1, 512), (3, 512), (8, 512), (5, 80)])  # 80 threads: no whole number of warps
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("n", [1, 7, 9, 15, 17, 23, 255, 257, 8 * 31 + 1, 8 * 33 + 7, 8 * 512 * 8 + 1, 8 * 512 * 8 * 3 + 13, 250001])
+def test_all_gather_slots_off_the_vector_grid(emu_worlds, W, block, dtype, n):
+    """Shards of any size: every alignment of a slot, the ends of warps, slabs and CTAs; nothing past the end is written."""
+    import tccl_b200 as tccl
+    from tccl_b200.parallel.emu import EmuTensor
+
+    w = emu_worlds(W)
+    x = make_inputs(w, W, n, dtype, 3100)
+    full = [torch.full((W * n + 64,), 77.0, dtype=dtype, device=w.device) for _ in range(W)]
+    old, w.config.block = w.config.block, block
+    try:
+        tccl.all_gather(x, out=EmuTensor([f[: W * n].view(W, n) for f in full]), algo="pull", world=w)
+        torch.cuda.synchronize()
+    finally:
+        w.config.block = old
+    w.check()
+    ref = torch.stack(list(x.parts))
+    for r in range(W):
+        assert torch.equal(full[r][: W * n].view(W, n), ref)
+        assert bool((full[r][W * n:] == 77.0).all())
+
+
 @pytest.mark.parametrize("W", [2, 4, 8])
 @pytest.mark.parametrize("n", [8, 1 << 12, (1 << 16) + 8])
 def test_all_gather_push(emu_worlds, W, n):
