@@ -51,14 +51,22 @@
 // slices (TCCL_TREE_SLICE_BYTES) and ONE fence.acq_rel.sys per slice followed by
 // relaxed stores of all the counters, instead of a st.release per counter.
 //
+// None of that protocol stands between two slices of a CTA: the data warps only load, add and store; one more
+// warp polls the counters up to kAhead slices ahead of them and another one fences and posts the counters behind
+// them, handing over through mbarriers in shared memory (ready: inputs there and destination free; done: every
+// data warp has issued its stores; sent: counters posted).  With one CTA-wide sequence poll - barrier - move -
+// barrier - fence - post, a slice cost 4 us on top of moving it (fp32, emulated: 8 MiB at 4 ranks 80 us, now 62;
+// 8 MiB at 8 ranks 162, now 122; 64 MiB at 4 ranks 333, now 296).
+//
 // The element count must be a whole number of 16-byte vectors (the reference
 // asks the same: triton_double_tree_allreduce.py:346-348).
-#include "common.cuh"
+#include "gemm_tcgen05.cuh"
 
 namespace tccl {
 
 constexpr int kTreeDepth = TCCL_TREE_RING_DEPTH;
 constexpr uint64_t kTreeSlice = TCCL_TREE_SLICE_BYTES;
+constexpr int kTreeCtrl = 64;  // threads of a CTA that poll and post the counters, beside up to 448 that move data
 
 __host__ __device__ __forceinline__ int tree_max_ctas(uint64_t tree_bytes) {
   if (tree_bytes < TCCL_TREE_LL_BYTES) return 0;  // the small-message part comes first
@@ -69,7 +77,8 @@ __host__ __device__ __forceinline__ int tree_max_ctas(uint64_t tree_bytes) {
 template <typename T, bool kPullDown>
 struct TreeAllReduce {
   using Args = tccl_tree_args;
-  static constexpr int kMaxThreads = 512, kMinBlocks = 1;
+  static constexpr int kMaxThreads = 512, kMinBlocks = 1;  // (576 would leave 96 registers a thread: spills)
+  static constexpr int kAhead = 4;  // slices between polling and posting
   static constexpr int U = 4;  // vectors in flight per thread and source
 
   static __device__ __forceinline__ uint32_t* up_flag(const tccl_comm& c, int rank, int tree, int k, int slot) {
@@ -110,136 +119,175 @@ struct TreeAllReduce {
     char* lres = left >= 0 ? reinterpret_cast<char*>(a.buf[left]) : nullptr;
     char* rres = right >= 0 ? reinterpret_cast<char*>(a.buf[right]) : nullptr;
     char* out = reinterpret_cast<char*>(a.out);
-    const int t = threadIdx.x, nt = blockDim.x;
+    const int t = threadIdx.x, nt = (int)blockDim.x - kTreeCtrl, lane = t & 31;  // nt data threads, whole warps
     uint32_t* seq_word = c.local + TCCL_LOCAL_TREE_SEQ + role * TCCL_TREE_MAX_CTAS + k;
     const uint32_t base = *seq_word;  // chunks this pipeline has moved in earlier calls
     const int cslot = a.child_slot[tree];
 
-    bool ok = true;
-    if (is_up) {
-      for (uint64_t n = 0; n < mine && ok; ++n) {
-        const uint32_t g = base + (uint32_t)n;  // running chunk number of this pipeline
-        // the children's partials are in my ring; the slot I am about to fill at the parent is free
-        if (t < 2) {
-          const int kid = t == 0 ? left : right;
-          if (kid >= 0) ok = wait_reach(up_flag(c, me, tree, k, t), g + 1u, c, deadline, kid, TCCL_W_TREE_UP);
-        } else if (t == 2 && parent >= 0) {
-          ok = wait_reach(ack_flag(c, me, tree, k), g + 1u - (uint32_t)kTreeDepth, c, deadline, parent, TCCL_W_TREE_UP);
-        }
-        ok = __syncthreads_and(ok);
-        if (!ok) break;
-        const uint64_t clo = (2 * n + tree) * cv, chi = min(clo + cv, nvec);
-        const uint64_t per = (chi - clo + K - 1) / K, lo = min(clo + per * k, chi), hi = min(lo + per, chi);
-        const char* lring = left >= 0 ? ring(c, me, tree, 0, k, g) : nullptr;
-        const char* rring = right >= 0 ? ring(c, me, tree, 1, k, g) : nullptr;
-        char* pring = parent >= 0 ? ring(c, parent, tree, cslot, k, g) : nullptr;
-        for (uint64_t i0 = lo + t; i0 < hi; i0 += (uint64_t)U * nt) {
-          Vec16 vo[U], vl[U], vr[U];
-#pragma unroll
-          for (int u = 0; u < U; ++u) {
-            const uint64_t i = i0 + (uint64_t)u * nt;
-            if (i < hi) {
-              vo[u] = ld_peer(in + i * 16);
-              if (lring) vl[u] = ld_peer(lring + (i - lo) * 16);
-              if (rring) vr[u] = ld_peer(rring + (i - lo) * 16);
-            }
-          }
-#pragma unroll
-          for (int u = 0; u < U; ++u) {
-            const uint64_t i = i0 + (uint64_t)u * nt;
-            if (i < hi) {
-              Vec16 r = vo[u];
-              if (lring) {
-                Acc<T> acc;
-                acc.zero();
-                acc.add(vo[u]);
-                acc.add(vl[u]);
-                if (rring) acc.add(vr[u]);
-                r = acc.pack();
-              }
-              if (pring) {
-                st_peer(pring + (i - lo) * 16, r);
-              } else {  // the root: this is the final value
-                st_peer(res + i * 16, r);
-                if (!kPullDown) {
-                  if (lres) st_peer(lres + i * 16, r);
-                  if (rres) st_peer(rres + i * 16, r);
-                }
-                if (out) st_local(out + i * 16, r);
-              }
-            }
-          }
-        }
-        __syncthreads();  // every thread has used what it loaded and issued its stores
-        if (t == 0) {
+    __shared__ uint64_t s_ready[kAhead], s_done[kAhead], s_sent[kAhead];
+    __shared__ int s_abort;
+    if (t == 0) {
+      s_abort = 0;
+      for (int i = 0; i < kAhead; ++i) {
+        gemm::mbar_init(s_ready + i, 1);
+        gemm::mbar_init(s_done + i, nt / 32);
+        gemm::mbar_init(s_sent + i, 1);
+      }
+      gemm::fence_barrier_init();
+    }
+    __syncthreads();
+    // a wait inside the CTA ends at the latest some time after the counters' deadline, whose miss is the one to report
+    const gemm::Abort ab{&s_abort, &c, status_of(c), deadline + c.timeout_ns / 4 + 1000000ull};
+    const uint64_t slices = is_up || parent >= 0 ? mine : 0;  // the root has no way down
+
+    if (t >= nt + 32) {
+      // ------------------------------------------------------------------ posting warp
+      if (lane == 0) {
+        for (uint64_t n = 0; n < slices; ++n) {
+          const uint32_t g = base + (uint32_t)n;
+          const int i = (int)(n % kAhead);
+          if (!gemm::mbar_wait(s_done + i, (uint32_t)(n / kAhead) & 1u, ab)) break;
           // ONE release fence (it waits until the CTA's stores have been performed; a per-flag
           // st.release would pay that once per flag), then the counters as relaxed stores
           fence_acq_rel_sys();
-          if (parent >= 0) {
+          if (is_up && parent >= 0) {
             st_relaxed_sys(up_flag(c, parent, tree, k, cslot), g + 1u);
           } else {
             if (left >= 0) st_relaxed_sys(down_flag(c, left, tree, k), g + 1u);
             if (right >= 0) st_relaxed_sys(down_flag(c, right, tree, k), g + 1u);
           }
-          if (left >= 0) st_relaxed_sys(ack_flag(c, left, tree, k), g + 1u);
-          if (right >= 0) st_relaxed_sys(ack_flag(c, right, tree, k), g + 1u);
+          if (is_up) {
+            if (left >= 0) st_relaxed_sys(ack_flag(c, left, tree, k), g + 1u);
+            if (right >= 0) st_relaxed_sys(ack_flag(c, right, tree, k), g + 1u);
+          } else if (kPullDown) {  // this slice of the parent's buffer is no longer needed
+            st_relaxed_sys(dack_flag(c, parent, tree, k, cslot), g + 1u);
+          }
+          gemm::mbar_arrive(s_sent + i);
         }
       }
-    } else {
-      const char* pres = parent >= 0 ? reinterpret_cast<const char*>(a.buf[parent]) : nullptr;
-      for (uint64_t n = 0; parent >= 0 && n < mine && ok; ++n) {
+    } else if (t >= nt) {
+      // ------------------------------------------------------------------ polling warp
+      bool ok = true;
+      for (uint64_t n = 0; n < slices && ok; ++n) {
         const uint32_t g = base + (uint32_t)n;
-        if (t == 0) ok = wait_reach(down_flag(c, me, tree, k), g + 1u, c, deadline, parent, TCCL_W_TREE_DOWN);
-        ok = __syncthreads_and(ok);
-        if (!ok) break;
-        if (kPullDown || lres || out) {
-          const uint64_t clo = (2 * n + tree) * cv, chi = min(clo + cv, nvec);
-          const uint64_t per = (chi - clo + K - 1) / K, lo = min(clo + per * k, chi), hi = min(lo + per, chi);
-          constexpr int UD = 8;
-          // pull: the slice is in the PARENT's result buffer; push: it is already in the own one
-          const char* src = kPullDown ? pres : res;
-          for (uint64_t i0 = lo + t; i0 < hi; i0 += (uint64_t)UD * nt) {
-            Vec16 v[UD];
+        const int i = (int)(n % kAhead);
+        if (n >= kAhead) ok = gemm::mbar_wait(s_sent + i, (uint32_t)(n / kAhead - 1) & 1u, ab);
+        if (is_up) {
+          // the children's partials are in my ring; the slot to be filled at the parent is free
+          if (ok && lane < 2) {
+            const int kid = lane == 0 ? left : right;
+            if (kid >= 0) ok = wait_reach(up_flag(c, me, tree, k, lane), g + 1u, c, deadline, kid, TCCL_W_TREE_UP);
+          } else if (ok && lane == 2 && parent >= 0) {
+            ok = wait_reach(ack_flag(c, me, tree, k), g + 1u - (uint32_t)kTreeDepth, c, deadline, parent, TCCL_W_TREE_UP);
+          }
+        } else if (ok && lane == 0) {
+          ok = wait_reach(down_flag(c, me, tree, k), g + 1u, c, deadline, parent, TCCL_W_TREE_DOWN);
+        }
+        ok = __all_sync(0xffffffffu, ok);
+        __syncwarp();  // the lanes' acquires come before lane 0's arrival
+        if (lane == 0) {
+          if (ok) gemm::mbar_arrive(s_ready + i);
+          else *(volatile int*)&s_abort = 1;
+        }
+        __syncwarp();
+      }
+      if (kPullDown && !is_up && ok && mine) {
+        // nobody may still be loading from this rank's result buffer when the kernel returns
+        if (lane < 2) {
+          const int kid = lane == 0 ? left : right;
+          if (kid >= 0)
+            ok = wait_reach(dack_flag(c, me, tree, k, lane), base + (uint32_t)mine, c, deadline, kid, TCCL_W_TREE_DOWN);
+        }
+        if (!ok) *(volatile int*)&s_abort = 1;
+      }
+    } else {
+      // -------------------------------------------------------------------- data warps
+      const char* pres = parent >= 0 ? reinterpret_cast<const char*>(a.buf[parent]) : nullptr;
+      const bool moves = is_up || kPullDown || lres || out;  // a leaf without `out` has its result in place already
+      for (uint64_t n = 0; n < slices; ++n) {
+        const uint32_t g = base + (uint32_t)n;
+        const int si = (int)(n % kAhead);
+        if (!gemm::mbar_wait(s_ready + si, (uint32_t)(n / kAhead) & 1u, ab)) break;
+        const uint64_t clo = (2 * n + tree) * cv, chi = min(clo + cv, nvec);
+        const uint64_t per = (chi - clo + K - 1) / K, lo = min(clo + per * k, chi), hi = min(lo + per, chi);
+        // pointers to the slice and 32-bit offsets: 64-bit element numbers cost the registers of the loads
+        const uint32_t bytes = (uint32_t)(hi - lo) * 16, st = (uint32_t)nt * 16;
+        char* sres = res + lo * 16;
+        char* slres = lres ? lres + lo * 16 : nullptr;
+        char* srres = rres ? rres + lo * 16 : nullptr;
+        char* sout = out ? out + lo * 16 : nullptr;
+        if (is_up) {
+          const char* sin = in + lo * 16;
+          const char* lring = left >= 0 ? ring(c, me, tree, 0, k, g) : nullptr;
+          const char* rring = right >= 0 ? ring(c, me, tree, 1, k, g) : nullptr;
+          char* pring = parent >= 0 ? ring(c, parent, tree, cslot, k, g) : nullptr;
+          for (uint32_t i0 = (uint32_t)t * 16; i0 < bytes; i0 += U * st) {
+            Vec16 vo[U], vl[U], vr[U];
 #pragma unroll
-            for (int u = 0; u < UD; ++u) {
-              const uint64_t i = i0 + (uint64_t)u * nt;
-              if (i < hi) v[u] = ld_peer(src + i * 16);
+            for (int u = 0; u < U; ++u) {
+              const uint32_t i = i0 + u * st;
+              if (i < bytes) {
+                vo[u] = ld_peer(sin + i);
+                if (lring) vl[u] = ld_peer(lring + i);
+                if (rring) vr[u] = ld_peer(rring + i);
+              }
             }
 #pragma unroll
-            for (int u = 0; u < UD; ++u) {
-              const uint64_t i = i0 + (uint64_t)u * nt;
-              if (i < hi) {
-                if (kPullDown) {
-                  st_peer(res + i * 16, v[u]);  // own buffer: the children pull it from here
-                } else {
-                  if (lres) st_peer(lres + i * 16, v[u]);
-                  if (rres) st_peer(rres + i * 16, v[u]);
+            for (int u = 0; u < U; ++u) {
+              const uint32_t i = i0 + u * st;
+              if (i < bytes) {
+                Vec16 r = vo[u];
+                if (lring) {
+                  Acc<T> acc;
+                  acc.zero();
+                  acc.add(vo[u]);
+                  acc.add(vl[u]);
+                  if (rring) acc.add(vr[u]);
+                  r = acc.pack();
                 }
-                if (out) st_local(out + i * 16, v[u]);
+                if (pring) {
+                  st_peer(pring + i, r);
+                } else {  // the root: this is the final value
+                  st_peer(sres + i, r);
+                  if (!kPullDown) {
+                    if (slres) st_peer(slres + i, r);
+                    if (srres) st_peer(srres + i, r);
+                  }
+                  if (sout) st_local(sout + i, r);
+                }
               }
             }
           }
-          __syncthreads();  // every thread's loads are complete (their values were stored) and its stores issued
-          if (t == 0) {
-            fence_acq_rel_sys();
-            if (left >= 0) st_relaxed_sys(down_flag(c, left, tree, k), g + 1u);
-            if (right >= 0) st_relaxed_sys(down_flag(c, right, tree, k), g + 1u);
-            // pull: this slice of the parent's buffer is no longer needed
-            if (kPullDown) st_relaxed_sys(dack_flag(c, parent, tree, k, cslot), g + 1u);
+        } else if (moves) {
+          constexpr int UD = 8;
+          // pull: the slice is in the PARENT's result buffer; push: it is already in the own one
+          const char* src = kPullDown ? pres + lo * 16 : sres;
+          for (uint32_t i0 = (uint32_t)t * 16; i0 < bytes; i0 += UD * st) {
+            Vec16 v[UD];
+#pragma unroll
+            for (int u = 0; u < UD; ++u)
+              if (i0 + u * st < bytes) v[u] = ld_peer(src + i0 + u * st);
+#pragma unroll
+            for (int u = 0; u < UD; ++u) {
+              const uint32_t i = i0 + u * st;
+              if (i < bytes) {
+                if (kPullDown) {
+                  st_peer(sres + i, v[u]);  // own buffer: the children pull it from here
+                } else {
+                  if (slres) st_peer(slres + i, v[u]);
+                  if (srres) st_peer(srres + i, v[u]);
+                }
+                if (sout) st_local(sout + i, v[u]);
+              }
+            }
           }
         }
-      }
-      if (kPullDown && ok && mine) {
-        // nobody may still be loading from this rank's result buffer when the kernel returns
-        if (t < 2) {
-          const int kid = t == 0 ? left : right;
-          if (kid >= 0)
-            ok = wait_reach(dack_flag(c, me, tree, k, t), base + (uint32_t)mine, c, deadline, kid, TCCL_W_TREE_DOWN);
-        }
-        ok = __syncthreads_and(ok);
+        __syncwarp();  // every lane has used what it loaded and issued its stores
+        if (lane == 0) gemm::mbar_arrive(s_done + si);
       }
     }
-    if (ok && t == 0) *seq_word = base + (uint32_t)mine;
+    __syncthreads();
+    if (t == 0 && !*(volatile int*)&s_abort) *seq_word = base + (uint32_t)mine;
   }
 };
 
@@ -249,8 +297,13 @@ using namespace tccl;
 
 extern "C" int tccl_tree_max_ctas(uint64_t tree_bytes) { return tree_max_ctas(tree_bytes); }
 
-extern "C" int tccl_allreduce_tree(const tccl_comm* comm, const tccl_tree_args* args, const tccl_launch* l) {
+// launch->block: threads of a CTA; rounded to whole warps, at least one that moves data beside the two control warps
+extern "C" int tccl_allreduce_tree(const tccl_comm* comm, const tccl_tree_args* args, const tccl_launch* launch) {
   const int dtype = args->dtype;
+  if (launch->block <= 0 || launch->block > 512) return -TCCL_EINVAL;
+  tccl_launch rounded = *launch;
+  rounded.block = launch->block < kTreeCtrl + 32 ? kTreeCtrl + 32 : launch->block / 32 * 32;
+  const tccl_launch* l = &rounded;
   if (l->n_emu == 0) {
     const int K = args->ctas_per_role;
     if (K < 1 || K > tree_max_ctas(comm->tree_bytes) || l->grid != 4 * K) return -TCCL_ESIZE;

@@ -38,6 +38,7 @@ __all__ = ["double_tree_all_reduce"]
 
 _SLICE = K["TCCL_TREE_SLICE_BYTES"]
 _LL_SLOT = K["TCCL_TREE_LL_SLOT_BYTES"]
+_PASS = 448 * 4 * 16  # bytes that the data warps of a full CTA of the chunked kernel have in flight per source
 
 
 def _tree_grid(w: WorldBase, nbytes: int):
@@ -52,7 +53,15 @@ def _tree_grid(w: WorldBase, nbytes: int):
         k = max(1, min(kmax, chunk_bytes // 16))
         return k, chunk_bytes // 16
     k = max(1, min(kmax, per_tree // 32768))
-    slice_bytes = max(4096, min(_SLICE, per_tree // k // 4, cfg.tree_chunk_bytes // k))
+    if w.emulated:
+        # What a slice costs beyond its data is hidden behind the other slices' data, so short ones (a quick
+        # start of the pipeline) win: one to three passes of the data warps, about eight slices or more per
+        # pipeline.  8 MiB at 4 ranks: 62 us (77 with a quarter of the share per slice), 32 MiB at 2: 87 (99).
+        # Over NVLink the large slices below are what was measured.
+        passes = max(1, min(3, per_tree // k // _PASS // 8))
+        slice_bytes = max(4096, min(_PASS * passes, per_tree // k, cfg.tree_chunk_bytes // k))
+    else:
+        slice_bytes = max(4096, min(_SLICE, per_tree // k // 4, cfg.tree_chunk_bytes // k))
     slice_bytes = max(16, slice_bytes // 16 * 16)
     return k, k * slice_bytes // 16
 
