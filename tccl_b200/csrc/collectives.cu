@@ -119,7 +119,7 @@ struct AllReduceOneShotP2P {
   // one rank: the reduction is a copy; keep it lean so two CTAs fit an SM
   static constexpr int kMaxThreads = 512, kMinBlocks = W == 1 ? 2 : 1;
   static constexpr int kMaxW = W ? W : TCCL_MAX_WORLD;
-  static constexpr int U = W == 1 ? 8 : ((W == 0 || W >= 8) ? 2 : 4);  // vectors per thread per pass
+  static constexpr int U = W == 1 ? 8 : ((W == 0 || W >= 5) ? 2 : 4);  // vectors per thread per pass
   static __device__ void run(const tccl_comm& c, const Args& a, int bid, int nb) {
     Entry sync(c, a.flags, bid);
     const int world = WorldOf<W>::get(c);
@@ -299,7 +299,7 @@ struct AllReduceTwoShotP2P {
   using Args = tccl_coll_args;
   static constexpr int kMaxThreads = 512, kMinBlocks = 1;
   static constexpr int kMaxW = W ? W : TCCL_MAX_WORLD;
-  static constexpr int U = (W == 0 || W >= 8) ? 2 : 4;
+  static constexpr int U = (W == 0 || W >= 5) ? 2 : 4;
   static __device__ void run(const tccl_comm& c, const Args& a, int bid, int nb) {
     Entry sync(c, a.flags, bid);
     const int world = WorldOf<W>::get(c);
@@ -535,7 +535,7 @@ struct ReduceScatter {
   using Args = tccl_coll_args;
   static constexpr int kMaxThreads = 512, kMinBlocks = 1;
   static constexpr int kMaxW = W ? W : TCCL_MAX_WORLD;
-  static constexpr int U = kNvls ? 8 : ((W == 0 || W >= 8) ? 2 : 4);
+  static constexpr int U = kNvls ? 8 : ((W == 0 || W >= 5) ? 2 : 4);
   static __device__ void run(const tccl_comm& c, const Args& a, int bid, int nb) {
     Entry sync(c, a.flags, bid);
     const int world = WorldOf<W>::get(c);
@@ -580,13 +580,21 @@ struct ReduceScatter {
 };
 
 // ------------------------------------------------------------------ dispatchers
+// One instance per world size up to 8: with a run-time count the loads of all 16 possible ranks hold registers and
+// the sums wait behind predicates.  24 MiB of bf16 per rank, one-shot all-reduce / two-shot / reduce-scatter in us,
+// emulated: 3 ranks 54 / 34.5 / 26 run-time, 39 / 31.5 / 22.5 so; 5 ranks 100 / 56 / 32.5 and 79 / 55 / 31; 7 ranks
+// 153 / 75 / 38 and 110 / 75 / 38.
 template <template <typename, int> class Op>
 static int dispatch(const tccl_comm* comm, const tccl_coll_args* args, const tccl_launch* l, int world, int dtype) {
 #define TCCL_W(T)                                                         \
   switch (world) {                                                        \
     case 1: return launch_op<Op<T, 1>>(comm, args, l);                    \
     case 2: return launch_op<Op<T, 2>>(comm, args, l);                    \
+    case 3: return launch_op<Op<T, 3>>(comm, args, l);                    \
     case 4: return launch_op<Op<T, 4>>(comm, args, l);                    \
+    case 5: return launch_op<Op<T, 5>>(comm, args, l);                    \
+    case 6: return launch_op<Op<T, 6>>(comm, args, l);                    \
+    case 7: return launch_op<Op<T, 7>>(comm, args, l);                    \
     case 8: return launch_op<Op<T, 8>>(comm, args, l);                    \
     default: return launch_op<Op<T, 0>>(comm, args, l);                   \
   }
