@@ -19,6 +19,10 @@
 //                          the peer's barrier (two plain commits; no multicast).
 //   tmem_full[a] (each)    same: two commits when an accumulator is complete.
 //   tmem_empty[a] (leader) the 2 x 128 epilogue threads of both CTAs arrive.
+// Arrivals from the other CTA (its epilogue's on tmem_empty, the MMA thread's commits on the
+// peer's empty[s]) must have landed before a CTA leaves: the next CTA on the SM may own those
+// bytes.  Nobody reuses the last accumulators and stages, so the barrier's owner waits for their
+// last phases explicitly (drain_* below) before the pair's final, relaxed cluster barrier.
 // The last partial wave of a shape whose tile count is not a multiple of the
 // number of pairs is cut into 256 x 128 half tiles, so the tail costs half a
 // tile instead of a whole one.
@@ -48,8 +52,9 @@ __device__ __forceinline__ uint32_t cluster_ctarank() {
 __device__ __forceinline__ void cluster_sync() {
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
-// the pair leaves together: orders nothing but the lifetime of shared and tensor memory, so no release (a release
-// here waited ~1 us for the epilogue's global stores to be acknowledged)
+// The pair leaves together.  Relaxed (a release here waited ~1 us for the epilogue's global stores to be acknowledged):
+// it does NOT order remote shared-memory operations issued before it, so whoever owns a barrier that the other CTA
+// signals has waited for the last of those arrivals before it comes here.
 __device__ __forceinline__ void cluster_sync_relaxed() {
   asm volatile("barrier.cluster.arrive.relaxed.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
 }
@@ -262,6 +267,21 @@ __device__ __forceinline__ int b_rows_default(int nt, int half, int cta) {
   return nt * BN2 + (half == 2 ? 128 : 0) + cta * (half ? 64 : 128);
 }
 
+// Waits until a ring of `n` barriers that has been used `it` times is free again: all arrivals of its last uses have
+// landed.  They were all issued before this is called, except after a failed wait (!ok), when some may never come: then
+// 100 ms must do.  Misses are not reported: nothing that was computed depends on these.
+__device__ __forceinline__ void drain_ring(uint64_t* bars, int n, uint32_t it, bool ok, uint64_t timeout_ns) {
+  int quiet = 0;
+  Abort ab{&quiet, nullptr, nullptr, 0};
+  for (int j = 0; j < n; ++j, ++it) {
+    uint64_t* bar = bars + it % n;
+    const uint32_t parity = ((it / n) & 1) ^ 1;
+    if (mbar_try_wait(bar, parity)) continue;  // the rule; reading the timer costs more than this
+    if (!ab.deadline) ab.deadline = globaltimer() + (ok || timeout_ns < 100000000ull ? timeout_ns : 100000000ull);
+    mbar_wait(bar, parity, ab);
+  }
+}
+
 template <class Policy>
 __device__ void run_mainloop2(const Shape shp, Policy& pol, const tccl_comm* comm, uint64_t timeout_ns,
                               uint64_t* trace = nullptr) {
@@ -325,11 +345,12 @@ __device__ void run_mainloop2(const Shape shp, Policy& pol, const tccl_comm* com
           tma_load_2d_pair(sm.b[s], map_b, leader_full, kb * BK2, yb);
         }
       }
+      drain_ring(sm.empty, kStages2, it, ok, timeout_ns);  // the MMA thread's last commits are here
     }
   } else if (warp == 1 && leader) {
     // ------------------------------------------------------------ MMA issuer (leader only)
     if (elect_one()) {
-      uint32_t it = 0;
+      uint32_t it = 0, tiles = 0;
       bool ok = true;
       int mt, nt, half;
       const uint32_t peer_empty0 = mapa(smem_u32(sm.empty), 1), peer_tfull0 = mapa(smem_u32(sm.tmem_full), 1);
@@ -356,8 +377,10 @@ __device__ void run_mainloop2(const Shape shp, Policy& pol, const tccl_comm* com
         if (ok) {
           tc_commit2(smem_u32(sm.tmem_full + acc));  // accumulator complete: both epilogues may read
           tc_commit2(peer_tfull0 + (uint32_t)acc * 8);
+          ++tiles;
         }
       }
+      drain_ring(sm.tmem_empty, 2, tiles, ok, timeout_ns);  // both epilogues' last arrivals are here
     }
   } else if (warp >= kEpiWarp0) {
     // ------------------------------------------------------------ epilogue (both CTAs, own rows)
@@ -385,8 +408,8 @@ __device__ void run_mainloop2(const Shape shp, Policy& pol, const tccl_comm* com
   }
 
   // Neither CTA's shared memory or tensor memory may go away while the other can still signal
-  // or read it; a CTA that gave up waits here for its partner, which gives up at the same
-  // deadline at the latest.  Loads in flight were all counted on `full` barriers that the MMA
+  // or read it (the signals of the other CTA have landed: drained above); a CTA that gave up waits here
+  // for its partner, which gives up at the same deadline at the latest.  Loads in flight were all counted on `full` barriers that the MMA
   // thread (or nobody, after a failure) consumed; they have landed by the time both CTAs are here
   // unless a wait failed, in which case the deadline (seconds) has long outlasted any copy.
   tc_fence_before();

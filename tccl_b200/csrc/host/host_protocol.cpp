@@ -1127,3 +1127,118 @@ extern "C" int hp_selftest_tree_ll(int world, int numel, int calls, int depth) {
   for (auto& x : th) x.join();
   return bad.load();
 }
+
+// ---------------------------------------------------------------------------
+// Model of how a CTA pair ends (gemm_tcgen05_2cta.cuh, gemm_skinny.cu).  The epilogue of the second CTA arrives on the
+// leader's tmem_empty barriers and the leader's MMA thread commits to the second CTA's empty barriers; such remote
+// arrivals travel through an INTERCONNECT thread that delivers them later than they are issued.  Both CTAs then meet at
+// a cluster barrier that orders only their own threads, and what a CTA leaves behind is taken over by the next one
+// (`rounds` pairs run one after the other on the same two shared memories).  The accumulators and stages used last are
+// reused by nobody, so nothing in the mainloop waits for the arrivals that free them: `drain` = 1 (the kernels) waits for
+// their last phases before the cluster barrier; `drain` = 0 is the mistake, kept so that the sanitizer can be seen to
+// catch it: a late arrival hits the shared memory of the next CTA.
+namespace {
+struct PairSmem {
+  Mbar full[2], empty[2], tmem_full[2], tmem_empty[2];
+  uint32_t owner = 0;  // plain: which CTA's shared memory this is; every delivery looks at it
+};
+struct Interconnect {
+  struct Arrival {
+    PairSmem* at;
+    Mbar* bar;
+    uint32_t owner;
+  };
+  std::vector<Arrival> sent;
+  std::atomic<int> issued{0};
+  std::atomic<bool> stop{false};
+  std::atomic<int> strays{0};  // arrivals that found another CTA's shared memory
+  std::atomic_flag lock = ATOMIC_FLAG_INIT;
+  explicit Interconnect(size_t cap) : sent(cap) {}
+  void arrive(PairSmem* at, Mbar* bar, uint32_t owner) {
+    while (lock.test_and_set(std::memory_order_acquire)) std::this_thread::yield();
+    sent[(size_t)issued.load(std::memory_order_relaxed)] = Arrival{at, bar, owner};
+    issued.fetch_add(1, std::memory_order_release);
+    lock.clear(std::memory_order_release);
+  }
+  void run() {
+    for (int t = 0;;) {
+      if (t < issued.load(std::memory_order_acquire)) {
+        std::this_thread::sleep_for(std::chrono::microseconds(20));  // on its way
+        const Arrival a = sent[(size_t)t++];
+        if (a.at->owner != a.owner) strays.fetch_add(1);
+        a.bar->arrive();
+      } else if (stop.load(std::memory_order_acquire)) {
+        return;
+      } else {
+        std::this_thread::yield();
+      }
+    }
+  }
+};
+}  // namespace
+
+extern "C" int hp_selftest_pair_exit(int tiles, int rounds, int drain) {
+  if (tiles < 0 || tiles > 64 || rounds < 1 || rounds > 1000) return 100;
+  PairSmem sm[2];
+  Interconnect net((size_t)rounds * tiles * 4 + 4);
+  std::thread wire([&] { net.run(); });
+  KernelBoundary edge;
+  // a stray arrival leaves a barrier out of step: nobody waits on after one (or after ten seconds)
+  const auto give_up = clk::now() + std::chrono::seconds(10);
+  auto await = [&](const Mbar& b, uint32_t parity) {
+    while ((b.phase.load(std::memory_order_acquire) & 1u) == parity && !net.strays.load(std::memory_order_relaxed)) {
+      if (clk::now() > give_up) net.strays.fetch_add(1);
+      std::this_thread::yield();
+    }
+  };
+  auto cta = [&](int c, int role) {
+    int sense = 0;
+    for (int round = 1; round <= rounds && !net.strays.load(); ++round) {
+      if (c == 0 && role == 0)
+        for (PairSmem& s : sm) {  // the next pair's CTAs set up the shared memory they were given
+          s.owner = (uint32_t)round;
+          for (int i = 0; i < 2; ++i) {
+            s.full[i].init(2);
+            s.empty[i].init(1);
+            s.tmem_full[i].init(1);
+            s.tmem_empty[i].init(2);
+          }
+        }
+      edge.arrive_and_wait(6, sense, &net.strays);  // producer, MMA (or idle) and epilogue threads of both CTAs
+      const uint32_t own = (uint32_t)round;
+      auto parity = [](int use) { return ((uint32_t)use & 1u) ^ 1u; };  // of a ring of two, before its use / 2-th filling
+      if (role == 0) {  // producer: one stage per tile; the bytes of both CTAs are counted on the leader's barrier
+        for (int t = 0; t < tiles; ++t) {
+          await(sm[c].empty[t & 1], parity(t >> 1));
+          if (c == 0) sm[0].full[t & 1].arrive();
+          else net.arrive(&sm[0], &sm[0].full[t & 1], own);
+        }
+        for (int t = tiles; drain && t < tiles + 2; ++t) await(sm[c].empty[t & 1], parity(t >> 1));
+      } else if (role == 1 && c == 0) {  // the leader's MMA thread
+        for (int t = 0; t < tiles; ++t) {
+          await(sm[0].tmem_empty[t & 1], parity(t >> 1));
+          await(sm[0].full[t & 1], (uint32_t)(t >> 1) & 1u);
+          sm[0].empty[t & 1].arrive();
+          net.arrive(&sm[1], &sm[1].empty[t & 1], own);
+          sm[0].tmem_full[t & 1].arrive();
+          net.arrive(&sm[1], &sm[1].tmem_full[t & 1], own);
+        }
+        for (int t = tiles; drain && t < tiles + 2; ++t) await(sm[0].tmem_empty[t & 1], parity(t >> 1));
+      } else if (role == 2) {  // epilogue
+        for (int t = 0; t < tiles; ++t) {
+          await(sm[c].tmem_full[t & 1], (uint32_t)(t >> 1) & 1u);
+          if (c == 0) sm[0].tmem_empty[t & 1].arrive();
+          else net.arrive(&sm[0], &sm[0].tmem_empty[t & 1], own);
+        }
+      }
+      edge.arrive_and_wait(6, sense, &net.strays);  // both CTAs leave together
+    }
+  };
+  std::vector<std::thread> th;
+  for (int c = 0; c < 2; ++c)
+    for (int role = 0; role < 3; ++role) th.emplace_back(cta, c, role);
+  for (auto& x : th) x.join();
+  net.stop.store(true);
+  wire.join();
+  return net.strays.load() ? 1 : 0;
+}

@@ -12,6 +12,7 @@ extern "C" int hp_selftest_ag_pair(int world, int ctas, int row_tiles, int calls
 extern "C" int hp_selftest_rs_pair(int world, int ctas, int tiles_per_owner, int calls, int mode);
 extern "C" int hp_selftest_tree_ll(int world, int numel, int calls, int depth);
 extern "C" int hp_selftest_bulk(int world, int ctas, int chunk, int chunks_per_cta, int calls, int early_release);
+extern "C" int hp_selftest_pair_exit(int tiles, int rounds, int drain);
 
 int main(int argc, char** argv) {
   if (argc > 2 && std::strcmp(argv[1], "push-broken-variant") == 0) {
@@ -38,6 +39,12 @@ int main(int argc, char** argv) {
     std::printf("hp_selftest_bulk(broken variant) -> %d\n", rc);
     return rc;
   }
+  if (argc > 2 && std::strcmp(argv[1], "pair-exit-broken-variant") == 0) {
+    // a CTA pair that leaves without waiting for the arrivals on its way to it: expected to be reported
+    const int rc = hp_selftest_pair_exit(std::atoi(argv[2]), 50, 0);
+    std::printf("hp_selftest_pair_exit(broken variant) -> %d\n", rc);
+    return rc;
+  }
   const int world = argc > 1 ? std::atoi(argv[1]) : 4;
   const int numel = argc > 2 ? std::atoi(argv[2]) : 1 << 14;
   const int chunk = argc > 3 ? std::atoi(argv[3]) : 1 << 9;
@@ -61,6 +68,11 @@ int main(int argc, char** argv) {
   for (int depth = 1; depth <= 4; depth += 3) {
     rc = hp_selftest_tree_ll(world, 194, 60, depth);
     std::printf("hp_selftest_tree_ll(world=%d, depth=%d) -> %d\n", world, depth, rc);
+    if (rc) return rc;
+  }
+  for (int tiles = 0; tiles <= 5; ++tiles) {
+    rc = hp_selftest_pair_exit(tiles, 50, 1);
+    std::printf("hp_selftest_pair_exit(tiles=%d) -> %d\n", tiles, rc);
     if (rc) return rc;
   }
   rc = hp_selftest_rs_pair(world, 3, 5, 40, 0);

@@ -78,7 +78,7 @@ def test_protocol_is_race_free_under_thread_sanitizer(W):
     (deferred release, final phase, epoch hand-over across calls), the all-gather -> GEMM arrival
     flags, the push all-reduce with changing sizes and grids, the barrier-free CTA-pair forms of both
     fused GEMM ops (two alternating halves, 40 calls with the ranks drifting apart; batched and
-    ring-ordered movers) and the stage pipeline of the bulk-copy all-reduce."""
+    ring-ordered movers), the way a CTA pair ends and the stage pipeline of the bulk-copy all-reduce."""
     import subprocess
 
     from tccl_b200.utils import build as B
@@ -164,5 +164,24 @@ def test_thread_sanitizer_flags_a_single_staging_half_without_a_barrier():
     except RuntimeError as e:
         pytest.skip(str(e)[:200])
     r = subprocess.run([str(exe), "rs-pair-broken-variant", "4"], capture_output=True, text=True, timeout=300)
+    out = r.stdout + r.stderr
+    assert "ThreadSanitizer: data race" in out or r.returncode != 0, out[-2000:]
+
+
+@pytest.mark.parametrize("tiles", [1, 2, 5])
+def test_a_cta_pair_that_leaves_before_its_last_arrivals_have_landed_is_caught(tiles):
+    """The other CTA's last arrivals on a pair's barriers free accumulators and stages that nobody reuses, so only an
+    explicit wait at the end orders them before the CTA's shared memory passes to the next one; the cluster barrier at
+    the end is a relaxed one and does not.  The variant without that wait must be caught; the kernels' order runs clean
+    in test_protocol_is_race_free_under_thread_sanitizer."""
+    import subprocess
+
+    from tccl_b200.utils import build as B
+
+    try:
+        exe = B.build_host_tsan()
+    except RuntimeError as e:
+        pytest.skip(str(e)[:200])
+    r = subprocess.run([str(exe), "pair-exit-broken-variant", str(tiles)], capture_output=True, text=True, timeout=300)
     out = r.stdout + r.stderr
     assert "ThreadSanitizer: data race" in out or r.returncode != 0, out[-2000:]
