@@ -69,13 +69,16 @@ class Plan:
     A plan holds raw addresses, not the caller's ordinary tensors: an activation that was
     all-reduced once must stay free-able, or the caching allocator could never reuse its
     address and every call would plan (and pin) another one.  Tensors in symmetric memory
-    may be referenced: the communicator keeps those allocations alive anyway."""
+    may be referenced: the communicator keeps those allocations alive anyway.
+
+    Every call of one plan writes into the same argument structs, so from the first write to the
+    return of the launcher a call holds the communicator's lock."""
 
     __slots__ = ("go", "structs", "world", "result", "fresh", "custom")
 
     def __init__(self, world, go, args, result=None, fresh=None, custom=None):
         self.world, self.go, self.structs, self.result = world, go, list(args.values()), result
-        self.custom = custom  # a complete replacement of run(), for plans that do not fit the pattern
+        self.custom = custom  # a replacement of run() (with the lock held), for plans that do not fit the pattern
         # fresh = (shape, dtype, device): a new output tensor per local rank and call.  empty_strided takes
         # half the host time of empty (1.1 against 2.1 us).
         self.fresh = None if fresh is None else (fresh[0], _dense_strides(fresh[0]), fresh[1], fresh[2])
@@ -87,13 +90,15 @@ class Plan:
     def run(self, x=None, out=None):
         if self.fresh is not None:  # fresh local output(s) per call
             outs = self.outputs()
-            for a, o in zip(self.structs, outs):
-                a.out = o.data_ptr()
-            self.go()
+            with self.world.lock:
+                for a, o in zip(self.structs, outs):
+                    a.out = o.data_ptr()
+                self.go()
             return self.world.wrap(outs)
-        if self.custom is not None:
-            return self.custom(x, out)
-        self.go()
+        with self.world.lock:
+            if self.custom is not None:
+                return self.custom(x, out)
+            self.go()
         res = self.result
         return x if res is _X else (out if res is _OUT else res)
 
@@ -115,10 +120,11 @@ def _planned(w: WorldBase, key, build: Callable[..., Plan], *args) -> Plan:
     """The plan of ``key`` (which starts with the operator's name and the tensors' keys); any change of the
     configuration makes a new one."""
     key = (key, w.config.version)
-    p = w.plans.lookup(key)
-    if p is None:
-        p = build(w, *args)
-        w.plans.insert(key, p)
+    with w.lock:
+        p = w.plans.lookup(key)
+        if p is None:
+            p = build(w, *args)
+            w.plans.insert(key, p)
     return p
 
 
@@ -297,15 +303,14 @@ def _plan_all_reduce(w, x, out, inplace, algo, sync_exit) -> Plan:
         if inplace:
             # a one-shot result cannot land in the buffer peers are still reading: stage it
             def run_staged(x_, _out):
+                staged = {r: torch.empty_like(w.local(x_, r)) for r in args}
                 for r, a in args.items():
-                    tmp = torch.empty_like(w.local(x_, r))
-                    staged[r], a.out = tmp, tmp.data_ptr()
+                    a.out = staged[r].data_ptr()
                 go()
-                for r in args:
-                    w.local(x_, r).copy_(staged.pop(r))
+                for r, tmp in staged.items():
+                    w.local(x_, r).copy_(tmp)
                 return x_
 
-            staged = {}
             return Plan(w, go, args, custom=run_staged)
         if out is not None:
             for r, a in args.items():

@@ -47,7 +47,8 @@ def _trace_ptr(w: WorldBase, trace, r: int, grid: int) -> int:
 class FusedPlan:
     """A bound launch of a fused kernel: validated argument structs, one per local rank in one array, and the
     launcher.  Holds raw addresses, no tensors (see ``collectives.Plan``); ``fresh`` = (shape, strides) of the
-    output that a call allocates when the caller gives none."""
+    output that a call allocates when the caller gives none.  The structs are shared by all calls of the plan:
+    they are written and launched under one hold of the communicator's lock."""
 
     __slots__ = ("arr", "l", "call", "name", "fresh", "user", "views")
 
@@ -58,14 +59,9 @@ class FusedPlan:
         self.call = lambda: fn(*refs)
 
     def outputs(self, like):
-        """New outputs next to the tensors ``like``, written into the argument structs."""
+        """New outputs next to the tensors ``like``."""
         shape, strides = self.fresh
-        outs = []
-        for g, t in zip(self.arr, like):
-            o = torch.empty_strided(shape, strides, dtype=torch.bfloat16, device=t.device)
-            g.out = o.data_ptr()
-            outs.append(o)
-        return outs
+        return [torch.empty_strided(shape, strides, dtype=torch.bfloat16, device=t.device) for t in like]
 
     def go(self, w: WorldBase, device) -> None:
         self.l.stream = torch._C._cuda_getCurrentRawStream(device.index)
@@ -109,12 +105,13 @@ def gemm_reduce_scatter(a, bt, out=None, *, trace=None, variant: str = "auto", w
     key = ("gemm_rs", _tkeys(As), _tkeys(Bs), Os and _tkeys(Os), variant)
     p = _planned(w, key, _plan_gemm_rs, As, Bs, Os, variant)
     grid = p.l.grid
-    for i, r in enumerate(w.local_ranks):
-        p.arr[i].trace = _trace_ptr(w, trace, r, grid) if trace is not None else 0
-    handoff = _stage_handoff(w, p.user)
-    p.l.meta = K["TCCL_RS_SYNC_ENTRY"] if handoff and p.user == "gemm_rs_pair" else 0
     outs = Os if Os is not None else p.outputs(As)
-    p.go(w, As[0].device)
+    with w.lock:
+        for g, r, o in zip(p.arr, w.local_ranks, outs):
+            g.out, g.trace = o.data_ptr(), _trace_ptr(w, trace, r, grid)
+        handoff = _stage_handoff(w, p.user)
+        p.l.meta = K["TCCL_RS_SYNC_ENTRY"] if handoff and p.user == "gemm_rs_pair" else 0
+        p.go(w, As[0].device)
     if out is not None:
         return out
     return outs if w.emulated else outs[0]
@@ -259,14 +256,15 @@ def all_gather_gemm(a_shard, bt, a_full=None, out=None, *, comm_ctas: int = 0, s
     key = ("ag_gemm", _tkeys(As), _tkeys(Bs), Os and _tkeys(Os), None if a_full is None else w.tkey(a_full), opts)
     p = _planned(w, key, _plan_ag_gemm, As, Bs, a_full, Os, *opts)
     grid = p.l.grid
-    for i, r in enumerate(w.local_ranks):
-        p.arr[i].trace = _trace_ptr(w, trace, r, grid) if trace is not None else 0
     outs = Os if Os is not None else p.outputs(As)
-    p.go(w, As[0].device)
     seq = 0
-    if p.user == "ag_gemm_pair":  # mirrors the device's count of pair calls, which picks the half (see reset())
-        seq = w.__dict__.get("_ag_seq", 0)
-        w.__dict__["_ag_seq"] = seq + 1
+    with w.lock:
+        for g, r, o in zip(p.arr, w.local_ranks, outs):
+            g.out, g.trace = o.data_ptr(), _trace_ptr(w, trace, r, grid)
+        p.go(w, As[0].device)
+        if p.user == "ag_gemm_pair":  # mirrors the device's count of pair calls, which picks the half (see reset())
+            seq = w.__dict__.get("_ag_seq", 0)
+            w.__dict__["_ag_seq"] = seq + 1
     res = out if out is not None else (outs if w.emulated else outs[0])
     return res, (a_full if a_full is not None else p.views[seq % len(p.views)])
 
@@ -365,7 +363,8 @@ def all_reduce_bias_residual_rmsnorm(x, weight, bias=None, residual=None, eps: f
     key = ("arn", w.tkey(x), _tkeys(Ws), Bs and _tkeys(Bs), Rs and _tkeys(Rs), eps, None if out is None else w.tkey(out),
            want_res, None if given is None else w.tkey(given), algo)
     p = _planned(w, key, _plan_arn, x, Ws, Bs, Rs, eps, out, want_res, given, algo)
-    p.go(w, Ws[0].device)
+    with w.lock:
+        p.go(w, Ws[0].device)
     if out is None:
         out = p.views[0]
     return (out, p.views[1] if given is None else given) if want_res else out

@@ -38,8 +38,9 @@ def quantized_all_reduce(x, out=None, *, world: Optional[WorldBase] = None):
     xs = _locals(w, x)
     os_ = _locals(w, out) if out is not None else None
     p = _planned(w, ("fp8wire", _tkeys(xs), os_ and _tkeys(os_)), _plan_quantized, xs, os_)
-    _stage_handoff(w, "fp8wire")
-    res = p.run()
+    with w.lock:
+        _stage_handoff(w, "fp8wire")
+        res = p.run()
     return out if out is not None else res
 
 

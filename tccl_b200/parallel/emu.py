@@ -18,7 +18,7 @@ import torch
 
 from ..config import Config
 from ..utils import lib as L
-from .world import PlanCache, WorldBase, _status_dict, tree_ring_bytes
+from .world import WorldBase, _status_dict, tree_ring_bytes
 
 K = L.K
 
@@ -84,7 +84,7 @@ class EmuWorld(WorldBase):
         self._zero_tree_ll()
         self.local_states = [torch.zeros(K["TCCL_LOCAL_WORDS"], dtype=torch.int32, device=self.device) for _ in range(W)]
         self.ll_bytes = min(2 << 20, self._stage_bytes // 4)
-        self.plans = PlanCache(self.config.plan_cache_size)
+        self._start_plans()
         self.comms = (L.Comm * W)()  # host structs: they travel with every launch
         self._fill_comms()
 

@@ -23,6 +23,7 @@ is resolved once and cached.
 from __future__ import annotations
 
 import ctypes as C
+import threading
 from collections import OrderedDict
 from typing import Dict, List, Optional, Sequence
 
@@ -82,6 +83,13 @@ class WorldBase:
     launches: int = 0  # kernels of this library launched so far
     emulated: bool = False  # all ranks in this process, on one GPU
 
+    def _start_plans(self) -> None:
+        # The op wrappers cache their bound launches in `plans`.  A cached launch owns ONE set of argument structs, and a
+        # call through ctypes lets other host threads run: whoever writes into the structs holds `lock` until the
+        # launcher has read them.  (Re-entrant: a symmetric tensor may be given back by a finaliser meanwhile.)
+        self.plans = PlanCache(self.config.plan_cache_size)
+        self.lock = threading.RLock()
+
     # -- to be provided by subclasses
     @property
     def local_ranks(self) -> List[int]:
@@ -113,9 +121,9 @@ class WorldBase:
     def prepare(self, name: str, args_by_rank: Dict[int, C.Structure], grid: int, block: int,
                 dtype_code: int = 0):
         """Bind one kernel launch to its arguments; returns a zero-argument callable
-        that enqueues it on the current stream.  The caller may patch a field (an output
-        pointer) of ``args_by_rank``'s structs between calls; a world may replace the dict's
-        values by structs of its own, so they are looked up there again."""
+        that enqueues it on the current stream, to be called with ``lock`` held.  The caller may patch a
+        field (an output pointer) of ``args_by_rank``'s structs before a call, under the same hold of the
+        lock; a world may replace the dict's values by structs of its own, so they are looked up there again."""
         raise NotImplementedError
 
     def comm_ref(self):
@@ -124,7 +132,9 @@ class WorldBase:
 
     def launch(self, name: str, args_by_rank: Dict[int, C.Structure], grid: int, block: int,
                dtype_code: int = 0) -> None:
-        self.prepare(name, args_by_rank, grid, block, dtype_code)()
+        go = self.prepare(name, args_by_rank, grid, block, dtype_code)
+        with self.lock:
+            go()
 
     def empty(self, shape, dtype=torch.bfloat16):
         raise NotImplementedError
@@ -188,7 +198,7 @@ class RealWorld(WorldBase):
         except (AttributeError, TypeError):  # the function is gone or changed its signature: nothing to enable
             pass
         self._handles: Dict[int, tuple] = {}
-        self.plans = PlanCache(self.config.plan_cache_size)  # op wrappers cache their bound launches here
+        self._start_plans()
         # workspace = [flag region | staging area], one symmetric allocation
         self._flag_bytes = -(-K["TCCL_FLAG_WORDS"] * 4 // 65536) * 65536
         self._stage_bytes = int(self.config.stage_mb) << 20
@@ -257,8 +267,9 @@ class RealWorld(WorldBase):
 
     def free(self, t: torch.Tensor) -> None:
         """Forget a symmetric allocation (and every cached launch that points into it)."""
-        self._handles.pop(t.untyped_storage().data_ptr(), None)
-        self.plans.clear()
+        with self.lock:
+            self._handles.pop(t.untyped_storage().data_ptr(), None)
+            self.plans.clear()
 
     def handle(self, t: torch.Tensor):
         """The torch symmetric-memory handle of ``t``'s allocation."""
@@ -361,5 +372,6 @@ class RealWorld(WorldBase):
             if not hasattr(self.config, k):
                 raise AttributeError(k)
             setattr(self.config, k, v)
-        self.comm.timeout_ns = self.config.timeout_ns
-        self.plans.clear()
+        with self.lock:
+            self.comm.timeout_ns = self.config.timeout_ns
+            self.plans.clear()

@@ -1,0 +1,147 @@
+"""What cached launches share between calls, on the CPU with a stub in place of the native launchers: host threads that
+call one operator on the same operands, and what keeps a communicator alive."""
+import ctypes as C
+import sys
+import threading
+import time
+
+import pytest
+import torch
+
+from tccl_b200.config import Config
+from tccl_b200.ops import collectives, fused, quantized
+from tccl_b200.ops import tree_allreduce
+from tccl_b200.parallel.emu import EmuTensor, EmuWorld
+from tccl_b200.parallel.world import RealWorld
+from tccl_b200.utils import lib as L
+
+_here = threading.local()  # .stream: what the calling thread uses as its current stream
+
+
+class StubLib:
+    """The real library, but launchers only note what they were given: (name, outputs, stream).  Like a call through
+    ctypes they let other threads run before they look at the structs."""
+
+    def __init__(self, real):
+        self._real, self.seen = real, []
+
+    def __getattr__(self, name):
+        if "stage_bytes" in name or "chunk_bytes" in name or "max_ctas" in name or "error" in name:
+            return getattr(self._real, name)
+
+        def launch(*refs):
+            time.sleep(0)
+            args, l = refs[1]._obj, refs[-1]._obj
+            structs = list(args) if isinstance(args, C.Array) else [args]
+            self.seen.append((name, [s.out if isinstance(s.out, int) else s.out[r] for r, s in enumerate(structs)], l.stream or 0))
+            return 0
+
+        return launch
+
+
+@pytest.fixture
+def stub(monkeypatch):
+    s = StubLib(L.lib())
+    monkeypatch.setattr(L, "lib", lambda: s)
+    monkeypatch.setattr(torch._C, "_cuda_getCurrentRawStream", lambda dev: getattr(_here, "stream", 7), raising=False)
+    for m in (collectives, fused, tree_allreduce):
+        monkeypatch.setattr(m, "check_sym_tensor", lambda *a, **k: None)
+    return s
+
+
+def one_rank(stub):
+    """A one-rank communicator over ordinary CPU memory."""
+    class World(RealWorld):
+        def __init__(self):
+            self._test_setup()
+
+        def _resolve(self, t):
+            return [t.data_ptr()], 0
+
+        def empty(self, shape, dtype=torch.bfloat16):
+            return torch.empty(shape, dtype=dtype)
+
+        def _test_setup(self):
+            self.config = Config()
+            self.world_size, self.rank, self._nvls, self._sms = 1, 0, False, 148
+            self.device = torch.device("cuda", 0)
+            self.ll_bytes, self.comm, self._handles = 2 << 20, L.Comm(), {}
+            self._start_plans()
+
+    return World()
+
+
+def emulated(stub, W):
+    w = object.__new__(EmuWorld)
+    w.world_size, w.config, w._sms, w.device = W, Config(), 148, torch.device("cuda", 0)
+    w._stage_bytes, w.ll_bytes, w.tree_bytes = 64 << 20, 2 << 20, 0
+    w.comms = (L.Comm * W)()
+    w.empty = lambda shape, dtype=torch.bfloat16: EmuTensor([torch.empty(shape, dtype=dtype) for _ in range(W)])
+    w._start_plans()
+    return w
+
+
+def _two_threads(fn, calls=400):
+    """Outputs returned to two threads that call ``fn`` at the same time, each on a stream of its own."""
+    got, errors = [[], []], []
+    gate = threading.Barrier(2)
+
+    def body(k):
+        _here.stream = 100 + k
+        try:
+            gate.wait()
+            for _ in range(calls):
+                got[k].append(fn())
+        except BaseException as e:  # noqa: BLE001
+            errors.append(e)
+
+    old = sys.getswitchinterval()
+    sys.setswitchinterval(1e-5)
+    try:
+        ts = [threading.Thread(target=body, args=(k,)) for k in (0, 1)]
+        [t.start() for t in ts]
+        [t.join() for t in ts]
+    finally:
+        sys.setswitchinterval(old)
+    assert not errors, errors[0]
+    return got
+
+
+def _ptrs(y):
+    return [t.data_ptr() for t in (y if isinstance(y, (list, EmuTensor)) else [y])]
+
+
+def _bf16(*shape):
+    return torch.zeros(shape, dtype=torch.bfloat16)
+
+
+CALLS = {
+    "gemm_reduce_scatter": lambda w, ops: fused.gemm_reduce_scatter(ops["a"], ops["b"], world=w),
+    "all_gather_gemm": lambda w, ops: fused.all_gather_gemm(ops["a"], ops["b"], world=w)[0],
+    "quantized_all_reduce": lambda w, ops: quantized.quantized_all_reduce(ops["x"], world=w),
+    "all_reduce_bias_residual_rmsnorm": lambda w, ops: fused.all_reduce_bias_residual_rmsnorm(ops["n"], ops["g"], world=w),
+    "all_reduce": lambda w, ops: collectives.all_reduce(ops["x"], world=w),
+    "all_gather": lambda w, ops: collectives.all_gather(ops["x"], world=w),
+}
+
+
+def _operands(w):
+    W = w.world_size
+    shapes = {"a": (256 * W, 64), "b": (256, 64), "x": (4096,), "n": (4, 1024), "g": (1024,)}
+    if not w.emulated:
+        return {k: _bf16(*s) for k, s in shapes.items()}
+    return {k: EmuTensor([_bf16(*s) for _ in range(W)]) for k, s in shapes.items()}
+
+
+@pytest.mark.parametrize("world", ["one rank", "emulated"])
+@pytest.mark.parametrize("op", sorted(CALLS))
+def test_two_threads_never_share_a_launch(stub, op, world):
+    """Every output that a call hands out was given to a launch of its own, on the calling thread's stream."""
+    w = one_rank(stub) if world == "one rank" else emulated(stub, 2)
+    ops = _operands(w)
+    got = _two_threads(lambda: CALLS[op](w, ops))
+    seen = {(tuple(outs), stream) for _, outs, stream in stub.seen}
+    missing = [(k, y) for k in (0, 1) for y in got[k] if (tuple(_ptrs(y)), 100 + k) not in seen]
+    assert not missing, f"{len(missing)} of {len(got[0]) + len(got[1])} outputs were in no launch of their thread"
+    streams = [stream for _, _, stream in stub.seen]
+    assert [streams.count(100), streams.count(101)] == [len(got[0]), len(got[1])] and w.launches == len(streams)
