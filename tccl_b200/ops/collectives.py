@@ -64,7 +64,10 @@ _X, _OUT = "<the caller's input>", "<the caller's out>"  # Plan.result: hand bac
 
 
 class Plan:
-    """A bound launch.  ``run(x, out)`` enqueues it; ``x`` / ``out`` are the tensors of THIS call.
+    """A bound launch.  ``run(w, x, out)`` enqueues it; ``x`` / ``out`` are the tensors of THIS call.
+
+    It holds no reference to its communicator ``w``, which holds it: dropping the last reference to a
+    communicator must free its device memory at once, not when the cycle collector happens to run.
 
     A plan holds raw addresses, not the caller's ordinary tensors: an activation that was
     all-reduced once must stay free-able, or the caching allocator could never reuse its
@@ -74,11 +77,12 @@ class Plan:
     Every call of one plan writes into the same argument structs, so from the first write to the
     return of the launcher a call holds the communicator's lock."""
 
-    __slots__ = ("go", "structs", "world", "result", "fresh", "custom")
+    __slots__ = ("go", "structs", "result", "fresh", "custom")
 
-    def __init__(self, world, go, args, result=None, fresh=None, custom=None):
-        self.world, self.go, self.structs, self.result = world, go, list(args.values()), result
-        self.custom = custom  # a replacement of run() (with the lock held), for plans that do not fit the pattern
+    def __init__(self, go, args, result=None, fresh=None, custom=None):
+        self.go, self.structs, self.result = go, list(args.values()), result
+        # custom(w, x, out): a replacement of run() (with the lock held), for plans that do not fit the pattern
+        self.custom = custom
         # fresh = (shape, dtype, device): a new output tensor per local rank and call.  empty_strided takes
         # half the host time of empty (1.1 against 2.1 us).
         self.fresh = None if fresh is None else (fresh[0], _dense_strides(fresh[0]), fresh[1], fresh[2])
@@ -87,18 +91,20 @@ class Plan:
         shape, strides, dtype, dev = self.fresh
         return [torch.empty_strided(shape, strides, dtype=dtype, device=dev) for _ in self.structs]
 
-    def run(self, x=None, out=None):
+    def run(self, w, x=None, out=None):
         if self.fresh is not None:  # fresh local output(s) per call
             outs = self.outputs()
-            with self.world.lock:
+            with w.lock:
                 for a, o in zip(self.structs, outs):
                     a.out = o.data_ptr()
                 self.go()
-            return self.world.wrap(outs)
-        with self.world.lock:
+                w.launches += 1
+            return w.wrap(outs)
+        with w.lock:
             if self.custom is not None:
-                return self.custom(x, out)
+                return self.custom(w, x, out)
             self.go()
+            w.launches += 1
         res = self.result
         return x if res is _X else (out if res is _OUT else res)
 
@@ -216,7 +222,7 @@ def all_reduce(x, out=None, *, inplace: bool = False, algo: str = "auto", world:
 
         return double_tree_all_reduce(x, out=out, inplace=inplace, world=w)
     key = ("ar", w.tkey(x), None if out is None else w.tkey(out), inplace, algo, sync_exit)
-    return _planned(w, key, _plan_all_reduce, x, out, inplace, algo, sync_exit).run(x, out)
+    return _planned(w, key, _plan_all_reduce, x, out, inplace, algo, sync_exit).run(w, x, out)
 
 
 def _plan_push(w, x, out, inplace, algo) -> Plan:
@@ -248,15 +254,15 @@ def _plan_push(w, x, out, inplace, algo) -> Plan:
     if inplace:
         for r, a in args.items():
             a.out = locs[r].data_ptr()  # each vector is read (into the slots) before the barrier, written after
-        return Plan(w, go, args, result=_X)
+        return Plan(go, args, result=_X)
     if out is not None:
         for r, a in args.items():
             o = w.local(out, r)
             _check_out(o, locs[r])
             a.out = o.data_ptr()
-        return Plan(w, go, args, result=_OUT)
+        return Plan(go, args, result=_OUT)
     shape, dtype, dev = tuple(x0.shape), x0.dtype, x0.device  # no reference to the caller's tensor
-    return Plan(w, go, args, fresh=(shape, dtype, dev))
+    return Plan(go, args, fresh=(shape, dtype, dev))
 
 
 def _plan_all_reduce(w, x, out, inplace, algo, sync_exit) -> Plan:
@@ -302,24 +308,25 @@ def _plan_all_reduce(w, x, out, inplace, algo, sync_exit) -> Plan:
         go = w.prepare(_AR_KERNELS[algo], args, grid, block, dt)
         if inplace:
             # a one-shot result cannot land in the buffer peers are still reading: stage it
-            def run_staged(x_, _out):
+            def run_staged(w, x_, _out):
                 staged = {r: torch.empty_like(w.local(x_, r)) for r in args}
                 for r, a in args.items():
                     a.out = staged[r].data_ptr()
                 go()
+                w.launches += 1
                 for r, tmp in staged.items():
                     w.local(x_, r).copy_(tmp)
                 return x_
 
-            return Plan(w, go, args, custom=run_staged)
+            return Plan(go, args, custom=run_staged)
         if out is not None:
             for r, a in args.items():
                 o = w.local(out, r)
                 _check_out(o, w.local(x, r))
                 a.out = o.data_ptr()
-            return Plan(w, go, args, result=_OUT)
+            return Plan(go, args, result=_OUT)
         shape, dtype, dev = tuple(x0.shape), x0.dtype, x0.device
-        return Plan(w, go, args, fresh=(shape, dtype, dev))
+        return Plan(go, args, fresh=(shape, dtype, dev))
     # two-shot: destination must be symmetric
     if not sym_dst:
         raise ValueError("two-shot all-reduce writes into symmetric memory: pass inplace=True or a symmetric out")
@@ -346,7 +353,7 @@ def _plan_all_reduce(w, x, out, inplace, algo, sync_exit) -> Plan:
         cap = w.config.max_ctas or w.config.pipe_ctas
         grid = grid_for(w, per_slice, nr * 32, ur, cap=cap)
         debug_log(w, f"all_reduce {nbytes} B -> {algo}, grid {grid} x {block}, pipe bits {bits:#x}")
-        return Plan(w, w.prepare(_AR_KERNELS[algo], args, grid, block, dt | bits), args,
+        return Plan(w.prepare(_AR_KERNELS[algo], args, grid, block, dt | bits), args,
                     result=_X if inplace else _OUT)
     if algo == "twoshot_bulk_p2p":
         lib = L.lib()
@@ -356,14 +363,14 @@ def _plan_all_reduce(w, x, out, inplace, algo, sync_exit) -> Plan:
         cap = max(1, w.num_sms() // w.world_size) if w.emulated else w.num_sms()
         grid = grid_for(w, per_slice, chunk_vecs, 1, cap=min(cap, w.config.max_ctas or cap))
         debug_log(w, f"all_reduce {nbytes} B -> {algo}, grid {grid} x 256")
-        return Plan(w, w.prepare(_AR_KERNELS[algo], args, grid, 256, dt), args, result=_X if inplace else _OUT)
+        return Plan(w.prepare(_AR_KERNELS[algo], args, grid, 256, dt), args, result=_X if inplace else _OUT)
     if algo == "twoshot_nvls":
         cap = w.config.nvls_ctas if not w.config.max_ctas else None
         grid = grid_for(w, per_slice, block, 8, cap=cap)
     else:
         grid = grid_for(w, per_slice, block, 2 if w.world_size >= 8 else 4)
     debug_log(w, f"all_reduce {nbytes} B -> {algo}, grid {grid} x {block}")
-    return Plan(w, w.prepare(_AR_KERNELS[algo], args, grid, block, dt), args, result=_X if inplace else _OUT)
+    return Plan(w.prepare(_AR_KERNELS[algo], args, grid, block, dt), args, result=_X if inplace else _OUT)
 
 
 def _plan_staged_twoshot(w, x, out, sync_exit) -> Plan:
@@ -381,24 +388,26 @@ def _plan_staged_twoshot(w, x, out, sync_exit) -> Plan:
         for r in w.local_ranks:
             _check_out(w.local(out, r), w.local(x, r))
 
-        def run_out(_x, out_):
+        def run_out(w, _x, out_):
             inner.go()
+            w.launches += 1
             for r in w.local_ranks:
                 w.local(out_, r).view(-1).copy_(w.local(buf, r))
             return out_
 
-        return Plan(w, inner.go, {}, custom=run_out)
+        return Plan(inner.go, {}, custom=run_out)
 
     shape, dtype, dev = tuple(x0.shape), x0.dtype, x0.device
 
-    def run_fresh(_x, _out):  # a new output tensor per call, filled from the symmetric buffer
+    def run_fresh(w, _x, _out):  # a new output tensor per call, filled from the symmetric buffer
         inner.go()
+        w.launches += 1
         outs = [torch.empty(shape, dtype=dtype, device=dev) for _ in w.local_ranks]
         for r, o in zip(w.local_ranks, outs):
             o.view(-1).copy_(w.local(buf, r))
         return w.wrap(outs)
 
-    return Plan(w, inner.go, {}, custom=run_fresh)
+    return Plan(inner.go, {}, custom=run_fresh)
 
 
 def all_gather(x, out=None, *, algo: str = "auto", world: Optional[WorldBase] = None, sync_exit: bool = True):
@@ -412,7 +421,7 @@ def all_gather(x, out=None, *, algo: str = "auto", world: Optional[WorldBase] = 
     """
     w = get_world(world)
     key = ("ag", w.tkey(x), None if out is None else w.tkey(out), algo, sync_exit)
-    return _planned(w, key, _plan_all_gather, x, out, algo, sync_exit).run(x, out)
+    return _planned(w, key, _plan_all_gather, x, out, algo, sync_exit).run(w, x, out)
 
 
 def _plan_all_gather(w, x, out, algo, sync_exit) -> Plan:
@@ -443,9 +452,9 @@ def _plan_all_gather(w, x, out, algo, sync_exit) -> Plan:
                 o = w.local(out, r)
                 _check_out(o, w.local(x, r), x0.numel() * W)
                 a.out = o.data_ptr()
-            return Plan(w, go, args, result=_OUT)
+            return Plan(go, args, result=_OUT)
         shape = (W, *x0.shape)
-        return Plan(w, go, args, fresh=(shape, x0.dtype, x0.device))
+        return Plan(go, args, fresh=(shape, x0.dtype, x0.device))
     if algo not in ("push", "push_nvls"):
         raise ValueError(f"unknown all-gather algo {algo!r}")
     if not out_is_sym:
@@ -466,7 +475,7 @@ def _plan_all_gather(w, x, out, algo, sync_exit) -> Plan:
         a.mc_out = w.mc_ptr(out)
         args[r] = a
     name = "tccl_allgather_push_nvls" if algo == "push_nvls" else "tccl_allgather_push_p2p"
-    return Plan(w, w.prepare(name, args, grid_for(w, nvec, block, 4), block, dt), args, result=_OUT)
+    return Plan(w.prepare(name, args, grid_for(w, nvec, block, 4), block, dt), args, result=_OUT)
 
 
 def reduce_scatter(x, out=None, *, algo: str = "auto", world: Optional[WorldBase] = None, sync_exit: bool = True):
@@ -476,7 +485,7 @@ def reduce_scatter(x, out=None, *, algo: str = "auto", world: Optional[WorldBase
     16-byte vector width (``triton_reduce_scatter.py:102-104``)."""
     w = get_world(world)
     key = ("rs", w.tkey(x), None if out is None else w.tkey(out), algo, sync_exit)
-    return _planned(w, key, _plan_reduce_scatter, x, out, algo, sync_exit).run(x, out)
+    return _planned(w, key, _plan_reduce_scatter, x, out, algo, sync_exit).run(w, x, out)
 
 
 def _plan_reduce_scatter(w, x, out, algo, sync_exit) -> Plan:
@@ -506,8 +515,8 @@ def _plan_reduce_scatter(w, x, out, algo, sync_exit) -> Plan:
             o = w.local(out, r)
             _check_out(o, w.local(x, r), per)
             a.out = o.data_ptr()
-        return Plan(w, go, args, result=_OUT)
-    return Plan(w, go, args, fresh=((per,), x0.dtype, x0.device))
+        return Plan(go, args, result=_OUT)
+    return Plan(go, args, fresh=((per,), x0.dtype, x0.device))
 
 
 # ---- reference-named entry points -------------------------------------------

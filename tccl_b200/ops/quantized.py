@@ -40,7 +40,7 @@ def quantized_all_reduce(x, out=None, *, world: Optional[WorldBase] = None):
     p = _planned(w, ("fp8wire", _tkeys(xs), os_ and _tkeys(os_)), _plan_quantized, xs, os_)
     with w.lock:
         _stage_handoff(w, "fp8wire")
-        res = p.run()
+        res = p.run(w)
     return out if out is not None else res
 
 
@@ -70,4 +70,4 @@ def _plan_quantized(w, xs, os_) -> Plan:
     cps = -(-(n // QUANT_CHUNK) // W)
     grid = max(1, min(-(-cps // 8), 2 * w.max_ctas()))  # a CTA's 8 warps take 8 chunks at a time
     go = w.prepare("tccl_allreduce_fp8wire", args, grid, 256)
-    return Plan(w, go, args, fresh=None if os_ is not None else (tuple(x0.shape), x0.dtype, x0.device))
+    return Plan(go, args, fresh=None if os_ is not None else (tuple(x0.shape), x0.dtype, x0.device))

@@ -69,7 +69,7 @@ def _tree_grid(w: WorldBase, nbytes: int):
 def double_tree_all_reduce(tensor, out=None, *, inplace: bool = False, world: Optional[WorldBase] = None):
     w = get_world(world)
     key = ("tree", w.tkey(tensor), None if out is None else w.tkey(out), inplace)
-    return _planned(w, key, _plan, tensor, out, inplace).run(tensor, out)
+    return _planned(w, key, _plan, tensor, out, inplace).run(w, tensor, out)
 
 
 def _plan(w: WorldBase, x, out, inplace: bool) -> Plan:
@@ -121,11 +121,11 @@ def _plan(w: WorldBase, x, out, inplace: bool) -> Plan:
     pull = K["TCCL_TREE_PULL_DOWN"] if nbytes >= w.config.tree_pull_min_bytes else 0
     go = w.prepare("tccl_allreduce_tree", args, 4 * k, w.config.block, dt | pull)
     if out is not None:
-        return Plan(w, go, args, result=_OUT)
+        return Plan(go, args, result=_OUT)
     if inplace:
-        return Plan(w, go, args, result=_X)
+        return Plan(go, args, result=_X)
     shape, dtype, dev = tuple(x0.shape), x0.dtype, x0.device
-    return Plan(w, go, args, fresh=(shape, dtype, dev))
+    return Plan(go, args, fresh=(shape, dtype, dev))
 
 
 def _neighbours(a, W: int, r: int) -> None:
@@ -169,8 +169,8 @@ def _plan_ll(w: WorldBase, x, out, inplace: bool, x0, dt: int, nbytes: int) -> P
     block = 128 if nbytes <= 8192 else (256 if nbytes <= 65536 else 512)
     go = w.prepare("tccl_allreduce_tree_ll", args, 4 * k, block, dt)
     if out is not None:
-        return Plan(w, go, args, result=_OUT)
+        return Plan(go, args, result=_OUT)
     if inplace:
-        return Plan(w, go, args, result=_X)
+        return Plan(go, args, result=_X)
     shape, dtype, dev = tuple(x0.shape), x0.dtype, x0.device
-    return Plan(w, go, args, fresh=(shape, dtype, dev))
+    return Plan(go, args, fresh=(shape, dtype, dev))

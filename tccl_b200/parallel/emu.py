@@ -182,7 +182,6 @@ class EmuWorld(WorldBase):
             rc = fn(comms_ref, arr_ref, l_ref)
             if rc:
                 L.check(rc, name)
-            self.launches += 1
 
         return go
 

@@ -121,7 +121,8 @@ class WorldBase:
     def prepare(self, name: str, args_by_rank: Dict[int, C.Structure], grid: int, block: int,
                 dtype_code: int = 0):
         """Bind one kernel launch to its arguments; returns a zero-argument callable
-        that enqueues it on the current stream, to be called with ``lock`` held.  The caller may patch a
+        that enqueues it on the current stream, to be called with ``lock`` held; the caller counts it in
+        ``launches``.  It keeps no reference to the communicator, which keeps the cached launches.    The caller may patch a
         field (an output pointer) of ``args_by_rank``'s structs before a call, under the same hold of the
         lock; a world may replace the dict's values by structs of its own, so they are looked up there again."""
         raise NotImplementedError
@@ -135,6 +136,7 @@ class WorldBase:
         go = self.prepare(name, args_by_rank, grid, block, dtype_code)
         with self.lock:
             go()
+            self.launches += 1
 
     def empty(self, shape, dtype=torch.bfloat16):
         raise NotImplementedError
@@ -330,7 +332,6 @@ class RealWorld(WorldBase):
             rc = fn(comm_ref, a_ref, l_ref)
             if rc:
                 L.check(rc, name)
-            self.launches += 1
 
         go.keep = (a, l)  # the structs the references point into
         return go

@@ -1,9 +1,11 @@
 """What cached launches share between calls, on the CPU with a stub in place of the native launchers: host threads that
 call one operator on the same operands, and what keeps a communicator alive."""
 import ctypes as C
+import gc
 import sys
 import threading
 import time
+import weakref
 
 import pytest
 import torch
@@ -145,3 +147,31 @@ def test_two_threads_never_share_a_launch(stub, op, world):
     assert not missing, f"{len(missing)} of {len(got[0]) + len(got[1])} outputs were in no launch of their thread"
     streams = [stream for _, _, stream in stub.seen]
     assert [streams.count(100), streams.count(101)] == [len(got[0]), len(got[1])] and w.launches == len(streams)
+
+
+@pytest.mark.parametrize("world", ["one rank", "emulated"])
+def test_a_dropped_communicator_is_freed_at_once(stub, world):
+    """Cached launches do not keep their communicator (and its device memory) alive: no cycle for the collector to find."""
+    w = one_rank(stub) if world == "one rank" else emulated(stub, 2)
+    ops = _operands(w)
+    for _ in range(2):
+        for op in sorted(CALLS):
+            CALLS[op](w, ops)
+    x = ops["x"]
+    collectives.all_reduce(x, inplace=True, algo="oneshot_p2p", world=w)
+    w.config.oneshot_max_bytes = 16
+    w.config.push_max_bytes = 16
+    collectives.all_reduce(x, world=w)                                        # staged: a symmetric buffer, then a copy
+    collectives.all_reduce(x, out=_like(w, x), algo="oneshot_p2p", world=w)
+    gone, had_gc = weakref.ref(w), gc.isenabled()
+    gc.disable()
+    try:
+        del w
+        assert gone() is None
+    finally:
+        if had_gc:
+            gc.enable()
+
+
+def _like(w, x):
+    return EmuTensor([p.clone() for p in x.parts]) if w.emulated else x.clone()
