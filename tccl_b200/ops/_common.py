@@ -1,7 +1,7 @@
 """Helpers shared by the op wrappers: validation, grid sizing, default world."""
 from __future__ import annotations
 
-from typing import Optional
+from typing import List, Optional
 
 import torch
 
@@ -42,15 +42,18 @@ def dtype_code(dtype: torch.dtype) -> int:
         raise TypeError(f"unsupported dtype {dtype}; supported: bfloat16, float32, float16") from None
 
 
-def check_sym_tensor(world: WorldBase, x, what: str = "tensor") -> None:
+def check_sym_tensor(world: WorldBase, x, what: str = "tensor") -> List[int]:
+    """Raises unless ``x`` can be given to a kernel as a symmetric tensor; returns every rank's address of it."""
     t = world.local(x, world.local_ranks[0])
     if not t.is_cuda:
         raise ValueError(f"{what} must live on the GPU in symmetric memory")
     if not t.is_contiguous():
         raise ValueError(f"{what} must be contiguous")
-    for p in world.peer_ptrs(x):
+    ptrs = world.peer_ptrs(x)
+    for p in ptrs:
         if p % 16:
             raise ValueError(f"{what} must start on a 16-byte boundary on every rank (view offset {p % 16})")
+    return ptrs
 
 
 def grid_for(world: WorldBase, nvec: int, block: int, per_thread: int, cap: Optional[int] = None) -> int:

@@ -29,8 +29,10 @@ def _locals(w: WorldBase, x):
     return [x]  # a real world drives exactly one rank
 
 
-def _tkeys(ts) -> tuple:
-    return tuple([(t.data_ptr(), t.shape, t.stride(), t.dtype) for t in ts])
+def _layouts(ts) -> tuple:
+    """What a fused kernel's plan depends on in its ordinary operands: everything but the address, of which only the
+    alignment matters."""
+    return tuple([(t.shape, t.stride(), t.dtype, t.data_ptr() & 15) for t in ts])
 
 
 def _trace_ptr(w: WorldBase, trace, r: int, grid: int) -> int:
@@ -45,9 +47,11 @@ def _trace_ptr(w: WorldBase, trace, r: int, grid: int) -> int:
 
 
 class FusedPlan:
-    """A bound launch of a fused kernel: validated argument structs, one per local rank in one array, and the
-    launcher.  Holds raw addresses, no tensors (see ``collectives.Plan``); ``fresh`` = (shape, strides) of the
-    output that a call allocates when the caller gives none.  The structs are shared by all calls of the plan:
+    """A validated launch of a fused kernel for one layout of its operands: argument structs, one per local rank in
+    one array, and the launcher.  Every call writes the addresses of its own operands into the structs, so tensors
+    at new addresses cost what known ones do: 11 us of host time for the RMSNorm operator.  (Keyed on addresses it
+    was 9 on known ones and 30 on new ones, more than the 18 without any plan.)  ``fresh`` = (shape, strides) of the output that a call allocates when the caller gives none;
+    ``views``: buffers of the communicator's own that a call hands out.  The structs are shared by all calls of the plan:
     they are written and launched under one hold of the communicator's lock."""
 
     __slots__ = ("arr", "l", "call", "name", "fresh", "user", "views")
@@ -102,13 +106,14 @@ def gemm_reduce_scatter(a, bt, out=None, *, trace=None, variant: str = "auto", w
     w = get_world(world)
     As, Bs = _locals(w, a), _locals(w, bt)
     Os = _locals(w, out) if out is not None else None
-    key = ("gemm_rs", _tkeys(As), _tkeys(Bs), Os and _tkeys(Os), variant)
+    key = ("gemm_rs", _layouts(As), _layouts(Bs), Os and _layouts(Os), variant)
     p = _planned(w, key, _plan_gemm_rs, As, Bs, Os, variant)
     grid = p.l.grid
     outs = Os if Os is not None else p.outputs(As)
     with w.lock:
-        for g, r, o in zip(p.arr, w.local_ranks, outs):
-            g.out, g.trace = o.data_ptr(), _trace_ptr(w, trace, r, grid)
+        for g, r, x, b, o in zip(p.arr, w.local_ranks, As, Bs, outs):
+            g.a, g.bt, g.out = x.data_ptr(), b.data_ptr(), o.data_ptr()
+            g.trace = _trace_ptr(w, trace, r, grid)
         handoff = _stage_handoff(w, p.user)
         p.l.meta = K["TCCL_RS_SYNC_ENTRY"] if handoff and p.user == "gemm_rs_pair" else 0
         p.go(w, As[0].device)
@@ -148,8 +153,8 @@ def _plan_gemm_rs(w, As, Bs, Os, variant) -> FusedPlan:
     for i, (ar, br) in enumerate(zip(As, Bs)):
         if ar.stride(1) != 1 or br.stride(1) != 1:
             raise ValueError("operands must have a unit inner stride")
-        optr, ldo = (Os[i].data_ptr(), Os[i].stride(0)) if Os is not None else (0, N)
-        arr[i] = L.GemmRsArgs(ar.data_ptr(), br.data_ptr(), optr, M, N, Kr, ar.stride(0), br.stride(0), ldo, 0)
+        ldo = Os[i].stride(0) if Os is not None else N
+        arr[i] = L.GemmRsArgs(0, 0, 0, M, N, Kr, ar.stride(0), br.stride(0), ldo, 0)
     name = "tccl_gemm_reduce_scatter_pair" if pair else "tccl_gemm_reduce_scatter"
     return FusedPlan(w, name, arr, _gemm_ctas(w, pair), 256, (C.c_uint64(stage_bytes),), ((M // W, N), (N, 1)),
                      "gemm_rs_pair" if pair else "gemm_rs")
@@ -252,15 +257,21 @@ def all_gather_gemm(a_shard, bt, a_full=None, out=None, *, comm_ctas: int = 0, s
     w = get_world(world)
     As, Bs = _locals(w, a_shard), _locals(w, bt)
     Os = _locals(w, out) if out is not None else None
-    opts = (comm_ctas, swiglu, int(lsu_movers), variant)
-    key = ("ag_gemm", _tkeys(As), _tkeys(Bs), Os and _tkeys(Os), None if a_full is None else w.tkey(a_full), opts)
-    p = _planned(w, key, _plan_ag_gemm, As, Bs, a_full, Os, *opts)
+    opts = (a_full is None, comm_ctas, swiglu, int(lsu_movers), variant)
+    key = ("ag_gemm", _layouts(As), _layouts(Bs), Os and _layouts(Os), opts)
+    p = _planned(w, key, _plan_ag_gemm, As, Bs, Os, *opts)
     grid = p.l.grid
     outs = Os if Os is not None else p.outputs(As)
-    seq = 0
+    full_ptrs, mc, seq = None, 0, 0
+    if a_full is not None:
+        full_ptrs, mc = w.peer_ptrs(a_full), _ag_multicast(w, a_full, p.user == "ag_gemm_pair")
     with w.lock:
-        for g, r, o in zip(p.arr, w.local_ranks, outs):
-            g.out, g.trace = o.data_ptr(), _trace_ptr(w, trace, r, grid)
+        for g, r, x, b, o in zip(p.arr, w.local_ranks, As, Bs, outs):
+            g.a_shard, g.bt, g.out = x.data_ptr(), b.data_ptr(), o.data_ptr()
+            g.trace = _trace_ptr(w, trace, r, grid)
+            if full_ptrs is not None:
+                g.a_full[: len(full_ptrs)] = full_ptrs
+                g.mc_a_full = mc
         p.go(w, As[0].device)
         if p.user == "ag_gemm_pair":  # mirrors the device's count of pair calls, which picks the half (see reset())
             seq = w.__dict__.get("_ag_seq", 0)
@@ -269,7 +280,12 @@ def all_gather_gemm(a_shard, bt, a_full=None, out=None, *, comm_ctas: int = 0, s
     return res, (a_full if a_full is not None else p.views[seq % len(p.views)])
 
 
-def _plan_ag_gemm(w, As, Bs, a_full, Os, comm_ctas, swiglu, lsu_movers, variant) -> FusedPlan:
+def _ag_multicast(w, a_full, pair) -> int:
+    # two ranks: the switch would deliver every row to its sender too (twice the inbound bytes of a plain store)
+    return w.mc_ptr(a_full) if ((w.world_size > 2 and not w.config.ag_ring) or not pair) else 0
+
+
+def _plan_ag_gemm(w, As, Bs, Os, own_full, comm_ctas, swiglu, lsu_movers, variant) -> FusedPlan:
     W = w.world_size
     a0, b0 = As[0], Bs[0]
     if a0.dtype != torch.bfloat16 or b0.dtype != torch.bfloat16:
@@ -291,8 +307,8 @@ def _plan_ag_gemm(w, As, Bs, a_full, Os, comm_ctas, swiglu, lsu_movers, variant)
     # one rank: the last pair tile may hang over the end of the rows
     pair = (pair_ok or (W == 1 and variant == "auto")) and variant != "single"
     half_bytes = 0
-    views = None
-    if a_full is None:
+    views, full_ptrs, mc = None, (), 0
+    if own_full:
         cache = w.__dict__.setdefault("_ag_buffers", {})
         key = (M, Kd, pair)
         a_full = cache.get(key)
@@ -301,9 +317,7 @@ def _plan_ag_gemm(w, As, Bs, a_full, Os, comm_ctas, swiglu, lsu_movers, variant)
         half = a_full.half if w.emulated else a_full.__getitem__
         views = [half(0), half(1)] if pair else [a_full]
         half_bytes = M * Kd * 2 if pair else 0
-    full_ptrs = w.peer_ptrs(a_full)
-    # two ranks: the switch would deliver every row to its sender too (twice the inbound bytes of a plain store)
-    mc = w.mc_ptr(a_full) if ((W > 2 and not w.config.ag_ring) or not pair) else 0
+        full_ptrs, mc = w.peer_ptrs(a_full), _ag_multicast(w, a_full, pair)
     grid = _gemm_ctas(w, pair)
     if comm_ctas <= 0:
         # Few data movers: every mover CTA is an SM the GEMM does not get, and 8 movers
@@ -315,18 +329,16 @@ def _plan_ag_gemm(w, As, Bs, a_full, Os, comm_ctas, swiglu, lsu_movers, variant)
     for i, (r, ar, br) in enumerate(zip(w.local_ranks, As, Bs)):
         if ar.stride(1) != 1 or br.stride(1) != 1:
             raise ValueError("operands must have a unit inner stride")
-        optr, ldo = 0, n_out
+        ldo = n_out
         if Os is not None:
             o = Os[i]
             if o.shape != (M, n_out) or o.dtype != torch.bfloat16 or o.stride(1) != 1:
                 raise ValueError(f"out must be bf16 [{M}, {n_out}] with a unit inner stride")
-            optr, ldo = o.data_ptr(), o.stride(0)
+            ldo = o.stride(0)
         g = arr[i]
-        g.a_shard = ar.data_ptr()
         for q, v in enumerate(full_ptrs):
             g.a_full[q] = v
         g.mc_a_full = mc
-        g.bt, g.out = br.data_ptr(), optr
         g.m, g.n, g.k = M, N, Kd
         g.lda_shard, g.lda_full, g.ldb, g.ldo = ar.stride(0), Kd, br.stride(0), ldo
         g.comm_ctas = max(1, int(w.config.ag_batches)) if pair else comm_ctas  # pair kernel: batches of the mover phase
@@ -360,19 +372,33 @@ def all_reduce_bias_residual_rmsnorm(x, weight, bias=None, residual=None, eps: f
     given = residual_out if want_res and residual_out is not True else None
     Ws, Bs, Rs = _locals(w, weight), (_locals(w, bias) if bias is not None else None), \
         (_locals(w, residual) if residual is not None else None)
-    key = ("arn", w.tkey(x), _tkeys(Ws), Bs and _tkeys(Bs), Rs and _tkeys(Rs), eps, None if out is None else w.tkey(out),
-           want_res, None if given is None else w.tkey(given), algo)
-    p = _planned(w, key, _plan_arn, x, Ws, Bs, Rs, eps, out, want_res, given, algo)
+    # the caller's symmetric tensors: checked, and their addresses taken, on every call
+    xp, op, rp = [None if t is None else check_sym_tensor(w, t, what)
+                  for t, what in ((x, "input"), (out, "out"), (given, "residual_out"))]
+    x0, eps = w.local(x, w.local_ranks[0]), float(eps)
+    key = ("arn", x0.shape, x0.dtype, _layouts(Ws), Bs and _layouts(Bs), Rs and _layouts(Rs), eps, out is None, want_res,
+           given is None, algo)
+    p = _planned(w, key, _plan_arn, x0, Ws, Bs, Rs, eps, out is None, want_res, given is None, algo)
+    W = w.world_size
     with w.lock:
+        for i, a in enumerate(p.arr):
+            a.x[:W], a.mc_x = xp, w.mc_ptr(x)
+            if op is not None:
+                a.out[:W], a.mc_out = op, w.mc_ptr(out)
+            if rp is not None:
+                a.res_out[:W], a.mc_res_out = rp, w.mc_ptr(given)
+            a.weight = Ws[i].data_ptr()
+            if Bs is not None:
+                a.bias = Bs[i].data_ptr()
+            if Rs is not None:
+                a.residual = Rs[i].data_ptr()
         p.go(w, Ws[0].device)
     if out is None:
         out = p.views[0]
     return (out, p.views[1] if given is None else given) if want_res else out
 
 
-def _plan_arn(w, x, Ws, Bs, Rs, eps, out, want_res, given_res, algo) -> FusedPlan:
-    check_sym_tensor(w, x, "input")
-    x0 = w.local(x, w.local_ranks[0])
+def _plan_arn(w, x0, Ws, Bs, Rs, eps, own_out, want_res, own_res, algo) -> FusedPlan:
     if x0.dim() != 2:
         raise ValueError("x must be [tokens, hidden]")
     T, H = x0.shape
@@ -382,31 +408,24 @@ def _plan_arn(w, x, Ws, Bs, Rs, eps, out, want_res, given_res, algo) -> FusedPla
         raise ValueError(f"hidden must be a multiple of {vpt} and at most {512 * 4 * vpt}")
     cache = w.__dict__.setdefault("_arn_buffers", {})
 
-    def sym(tag, given):
-        if given is not None:
-            check_sym_tensor(w, given, tag)
-            return given
+    def sym(tag):
         key = (tag, T, H, x0.dtype)
         if key not in cache:
             cache[key] = w.empty((T, H), x0.dtype)
         return cache[key]
 
-    o_given = out is not None
-    out = sym("out", out)
-    res_out = sym("residual_out", given_res) if want_res else None
+    out = sym("out") if own_out else None
+    res_out = sym("residual_out") if want_res and own_res else None
     if algo == "auto":
         algo = "nvls" if w.has_nvls and w.world_size > 2 else "p2p"
     if algo == "nvls" and not w.has_nvls:
         raise RuntimeError("nvls variant needs NVLS multicast")
-    xp, op = w.peer_ptrs(x), w.peer_ptrs(out)
-    rp = w.peer_ptrs(res_out) if want_res else None
     arr = (L.ArnArgs * len(w.local_ranks))()
     for i, a in enumerate(arr):
-        for q in range(w.world_size):
-            a.x[q], a.out[q] = xp[q], op[q]
-            a.res_out[q] = rp[q] if rp else 0
-        a.mc_x, a.mc_out = w.mc_ptr(x), w.mc_ptr(out)
-        a.mc_res_out = w.mc_ptr(res_out) if want_res else 0
+        if out is not None:
+            a.out[: w.world_size], a.mc_out = w.peer_ptrs(out), w.mc_ptr(out)
+        if res_out is not None:
+            a.res_out[: w.world_size], a.mc_res_out = w.peer_ptrs(res_out), w.mc_ptr(res_out)
         for name, src in (("weight", Ws), ("bias", Bs), ("residual", Rs)):
             if src is None:
                 continue
@@ -415,7 +434,6 @@ def _plan_arn(w, x, Ws, Bs, Rs, eps, out, want_res, given_res, algo) -> FusedPla
                 raise ValueError(f"{name} must be contiguous, 16-byte aligned and of x's dtype")
             if tns.numel() != (T * H if name == "residual" else H):
                 raise ValueError(f"{name} has the wrong size")
-            setattr(a, name, tns.data_ptr())
         a.eps, a.tokens, a.hidden, a.dtype = float(eps), T, H, dt
         a.flags = w.coll_flags()
     rows = -(-T // w.world_size)
@@ -424,8 +442,7 @@ def _plan_arn(w, x, Ws, Bs, Rs, eps, out, want_res, given_res, algo) -> FusedPla
     batch = 1                                          # rows a CTA handles together (kernel's R)
     grid = max(1, min(-(-rows // batch), w.max_ctas() * per_sm, K["TCCL_MAX_BLOCKS"]))
     p = FusedPlan(w, "tccl_allreduce_bias_residual_rmsnorm", arr, grid, 512, (1 if algo == "nvls" else 0,))
-    # only the communicator's own buffers are kept (it keeps them anyway), never the caller's
-    p.views = (None if o_given else out, None if given_res is not None else res_out)
+    p.views = (out, res_out)
     return p
 
 

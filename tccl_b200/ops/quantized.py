@@ -19,8 +19,8 @@ import torch
 from ..parallel.world import WorldBase
 from ..utils import lib as L
 from ._common import get_world
-from .collectives import Plan, _planned
-from .fused import _locals, _stage_handoff, _tkeys
+from .collectives import _planned
+from .fused import FusedPlan, _layouts, _locals, _stage_handoff
 
 __all__ = ["quantized_all_reduce", "QUANT_CHUNK"]
 
@@ -37,14 +37,17 @@ def quantized_all_reduce(x, out=None, *, world: Optional[WorldBase] = None):
     w = get_world(world)
     xs = _locals(w, x)
     os_ = _locals(w, out) if out is not None else None
-    p = _planned(w, ("fp8wire", _tkeys(xs), os_ and _tkeys(os_)), _plan_quantized, xs, os_)
+    p = _planned(w, ("fp8wire", _layouts(xs), os_ and _layouts(os_)), _plan_quantized, xs, os_)
+    outs = os_ if os_ is not None else p.outputs(xs)
     with w.lock:
+        for g, t, o in zip(p.arr, xs, outs):
+            g.inp, g.out = t.data_ptr(), o.data_ptr()
         _stage_handoff(w, "fp8wire")
-        res = p.run(w)
-    return out if out is not None else res
+        p.go(w, w.device)
+    return out if out is not None else w.wrap(outs)
 
 
-def _plan_quantized(w, xs, os_) -> Plan:
+def _plan_quantized(w, xs, os_) -> FusedPlan:
     W = w.world_size
     x0 = xs[0]
     if x0.dtype != torch.bfloat16:
@@ -58,16 +61,10 @@ def _plan_quantized(w, xs, os_) -> Plan:
     have = (w.config.stage_mb << 20) - w.ll_bytes
     if need > have:
         raise ValueError(f"staging area too small: need {need >> 20} MiB, have {have >> 20} MiB (raise TCCL_STAGE_MB)")
-    args = {}
-    for i, r in enumerate(w.local_ranks):
-        optr = 0
-        if os_ is not None:
-            o = os_[i]
-            if o.dtype != torch.bfloat16 or o.numel() != n or not o.is_contiguous() or o.data_ptr() % 16:
-                raise ValueError("out must be a contiguous, 16-byte aligned bf16 tensor of the input's size")
-            optr = o.data_ptr()
-        args[r] = QarArgs(xs[i].data_ptr(), optr, n, 0)
+    for o in os_ or ():
+        if o.dtype != torch.bfloat16 or o.numel() != n or not o.is_contiguous() or o.data_ptr() % 16:
+            raise ValueError("out must be a contiguous, 16-byte aligned bf16 tensor of the input's size")
+    arr = (QarArgs * len(xs))(*[QarArgs(0, 0, n, 0) for _ in xs])
     cps = -(-(n // QUANT_CHUNK) // W)
     grid = max(1, min(-(-cps // 8), 2 * w.max_ctas()))  # a CTA's 8 warps take 8 chunks at a time
-    go = w.prepare("tccl_allreduce_fp8wire", args, grid, 256)
-    return Plan(go, args, fresh=None if os_ is not None else (tuple(x0.shape), x0.dtype, x0.device))
+    return FusedPlan(w, "tccl_allreduce_fp8wire", arr, grid, 256, fresh=(tuple(x0.shape), x0.stride()))

@@ -35,6 +35,7 @@ class StubLib:
             time.sleep(0)
             args, l = refs[1]._obj, refs[-1]._obj
             structs = list(args) if isinstance(args, C.Array) else [args]
+            self.structs = [type(s).from_buffer_copy(s) for s in structs]
             self.seen.append((name, [s.out if isinstance(s.out, int) else s.out[r] for r, s in enumerate(structs)], l.stream or 0))
             return 0
 
@@ -47,7 +48,7 @@ def stub(monkeypatch):
     monkeypatch.setattr(L, "lib", lambda: s)
     monkeypatch.setattr(torch._C, "_cuda_getCurrentRawStream", lambda dev: getattr(_here, "stream", 7), raising=False)
     for m in (collectives, fused, tree_allreduce):
-        monkeypatch.setattr(m, "check_sym_tensor", lambda *a, **k: None)
+        monkeypatch.setattr(m, "check_sym_tensor", lambda w, x, *a: w.peer_ptrs(x))
     return s
 
 
@@ -175,3 +176,54 @@ def test_a_dropped_communicator_is_freed_at_once(stub, world):
 
 def _like(w, x):
     return EmuTensor([p.clone() for p in x.parts]) if w.emulated else x.clone()
+
+
+@pytest.mark.parametrize("world", ["one rank", "emulated"])
+def test_fused_operators_plan_once_per_layout(stub, world):
+    """Operands at new addresses reach the launcher without a new plan; a layout that is refused stays refused after a
+    good one of the same shape was planned."""
+    w = one_rank(stub) if world == "one rank" else emulated(stub, 2)
+    W, ranks = w.world_size, w.local_ranks
+    fields = {"gemm_reduce_scatter": {"a": "a", "bt": "b"}, "all_gather_gemm": {"a_shard": "a", "bt": "b"},
+              "quantized_all_reduce": {"inp": "x"}, "all_reduce_bias_residual_rmsnorm": {"weight": "g", "x": "n"}}
+    keep = []  # new addresses, not reused ones
+    for op, names in fields.items():
+        sizes = set()
+        for _ in range(3):
+            ops = _operands(w)
+            keep.append(ops)
+            CALLS[op](w, ops)
+            sizes.add(len(w.plans))
+            for r, s in zip(ranks, stub.structs):
+                for f, k in names.items():
+                    got, want = getattr(s, f), [w.local(ops[k], q).data_ptr() for q in ranks]
+                    assert (got == want[r]) if isinstance(got, int) else (list(got)[:W] == want), (op, f)
+        assert len(sizes) == 1, f"{op}: {sizes} plans"
+    emu = lambda f: EmuTensor([f() for _ in range(W)]) if w.emulated else f()  # noqa: E731
+    off = lambda *shape: _bf16(8 + int(torch.tensor(shape).prod()))[1: 1 + int(torch.tensor(shape).prod())].view(shape)  # noqa: E731
+    with pytest.raises(ValueError):  # 2 bytes off the 16-byte grid
+        CALLS["quantized_all_reduce"](w, {"x": emu(lambda: off(4096))})
+    with pytest.raises(ValueError):
+        CALLS["quantized_all_reduce"](w, {"x": emu(lambda: _bf16(2, 8192)[:, :2048])})
+    with pytest.raises(ValueError):
+        CALLS["all_reduce_bias_residual_rmsnorm"](w, {"n": keep[0]["n"], "g": emu(lambda: off(1024))})
+    with pytest.raises(ValueError):
+        CALLS["gemm_reduce_scatter"](w, {"a": emu(lambda: _bf16(64, 256 * W).t()), "b": keep[0]["b"]})
+    with pytest.raises(TypeError):
+        CALLS["all_gather_gemm"](w, {"a": emu(lambda: torch.zeros(256 * W, 64, dtype=torch.float16)), "b": keep[0]["b"]})
+
+
+def test_fused_operators_write_the_callers_buffers(stub):
+    """Symmetric tensors that the caller passes reach the launcher at their addresses of this call."""
+    w = one_rank(stub)
+    for _ in range(2):
+        ops, y, res, full = _operands(w), _bf16(4, 1024), _bf16(4, 1024), _bf16(256, 64)
+        assert fused.all_reduce_bias_residual_rmsnorm(ops["n"], ops["g"], residual=ops["n"], out=y, residual_out=res, world=w) == (y, res)
+        s, = stub.structs
+        assert (s.out[0], s.res_out[0], s.residual, s.bias) == (y.data_ptr(), res.data_ptr(), ops["n"].data_ptr(), 0)
+        out, got = fused.all_gather_gemm(ops["a"], ops["b"], a_full=full, world=w)
+        s, = stub.structs
+        assert got is full and s.a_full[0] == full.data_ptr() and s.out == out.data_ptr()
+        fused.all_reduce_bias_residual_rmsnorm(ops["n"], ops["g"], world=w)
+        s, = stub.structs
+        assert s.residual == 0 and s.res_out[0] == 0
