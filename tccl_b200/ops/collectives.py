@@ -126,11 +126,13 @@ def _planned(w: WorldBase, key, build: Callable[..., Plan], *args) -> Plan:
     """The plan of ``key`` (which starts with the operator's name and the tensors' keys); any change of the
     configuration makes a new one."""
     key = (key, w.config.version)
-    with w.lock:
-        p = w.plans.lookup(key)
-        if p is None:
-            p = build(w, *args)
-            w.plans.insert(key, p)
+    p = w.plans.lookup(key)
+    if p is None:
+        with w.lock:
+            p = w.plans.lookup(key)  # another thread may have been first
+            if p is None:
+                p = build(w, *args)
+                w.plans.insert(key, p)
     return p
 
 

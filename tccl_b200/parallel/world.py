@@ -56,12 +56,18 @@ class PlanCache(OrderedDict):
         self.maxsize = max(1, int(maxsize))
 
     def lookup(self, key):
+        """Without a lock: another thread may evict the plan between the two steps, which only means that it
+        was about to be the oldest."""
         p = self.get(key)
         if p is not None:
-            self.move_to_end(key)
+            try:
+                self.move_to_end(key)
+            except KeyError:
+                pass
         return p
 
     def insert(self, key, plan):
+        """With the communicator's lock held."""
         self[key] = plan
         while len(self) > self.maxsize:
             self.popitem(last=False)

@@ -227,3 +227,18 @@ def test_fused_operators_write_the_callers_buffers(stub):
         fused.all_reduce_bias_residual_rmsnorm(ops["n"], ops["g"], world=w)
         s, = stub.structs
         assert s.residual == 0 and s.res_out[0] == 0
+
+
+def test_plan_cache_lookups_race_with_evictions():
+    """Lookups take no lock: a plan that goes away in the middle of one is no error."""
+    from tccl_b200.parallel.world import PlanCache
+
+    class Evicting(PlanCache):
+        def get(self, key):  # another thread evicts the plan between the two steps of a lookup
+            p = super().get(key)
+            self.pop(key, None)
+            return p
+
+    cache = Evicting(4)
+    cache.insert("a", 1)
+    assert cache.lookup("a") == 1 and cache.lookup("a") is None
