@@ -64,7 +64,7 @@ int launch_gemm_pair(const tccl_gemm_args* g, int grid, cudaStream_t stream, uin
   if (((uintptr_t)g->a | (uintptr_t)g->bt | (uintptr_t)g->c) & 15) return -TCCL_EALIGN;
   if (g->swiglu && (g->n % BN2)) return -TCCL_ESIZE;  // whole gate|up tiles only
   int rc = 0;
-  if (grid <= 0 && !trace && launch_gemm_skinny(g, stream, &rc)) return rc;
+  if (grid <= 0 && !trace && launch_gemm_skinny(g, stream, timeout_ns, &rc)) return rc;
   CUtensorMap ma, mb128, mb64;
   rc = make_tmap_bf16_kmajor(&ma, g->a, g->m, g->k, g->lda, 128);  // each CTA loads 128 rows of A ...
   if (rc) return rc;

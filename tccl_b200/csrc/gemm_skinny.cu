@@ -45,6 +45,7 @@ struct SkinnyArgs {
   int M, N, K, ldc;   // N: columns of C
   int swiglu;         // rows of Bt: 256-row blocks of 128 gate rows and the 128 matching up rows; C has half as many columns
   uint32_t* status;
+  uint64_t timeout_ns;  // bound of the kernel's waits together
 };
 
 __device__ __forceinline__ float4 ld_dsmem_f4(uint32_t cluster_addr) {
@@ -146,8 +147,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
   tc_fence_after();
   const uint32_t tmem = *tmem_ptr;
   grid_dependency_wait();
-  constexpr uint64_t kTimeoutNs = 2000000000ull;
-  Abort ab{abort_flag, nullptr, p.status, globaltimer() + kTimeoutNs};
+  Abort ab{abort_flag, nullptr, p.status, globaltimer() + p.timeout_ns};
 
   if (warp == 0 || warp == 3) {
     // ------------------------------------------------------ TMA producers: warp 0 loads rows of Bt, warp 3 tokens.  Two
@@ -261,7 +261,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
   // their way to this CTA's barriers: each lane looks at the last phase of one stage's (all landed long ago, unless a wait
   // failed; a thread that waited for one stage after the other where the loads end cost 1.5 us, this 0.2).
   if (CG == 2 && !leader && warp == 0 && lane < NS && lane < kb1 - kb0)
-    drain_ring(empty + lane, 1, (uint32_t)((kb1 - kb0 - 1 - lane) / NS + 1), !*ab.flag, kTimeoutNs);
+    drain_ring(empty + lane, 1, (uint32_t)((kb1 - kb0 - 1 - lane) / NS + 1), !*ab.flag, p.timeout_ns);
   __syncthreads();
   if (cl > 1) cluster_sync_relaxed();
   if (warp == 2) {
@@ -272,7 +272,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
 }
 
 template <int TN, int CG>
-static int launch_tn(const tccl_gemm_args* g, int splits, int per_sm, cudaStream_t stream) {
+static int launch_tn(const tccl_gemm_args* g, int splits, int per_sm, uint64_t timeout_ns, cudaStream_t stream) {
   using Cfg = SkinnyCfg<TN, CG>;
   CUtensorMap mw, ma;
   int rc = make_tmap_bf16_kmajor(&mw, g->bt, g->n, g->k, g->ldb, g->swiglu ? 64 : 128);
@@ -287,27 +287,28 @@ static int launch_tn(const tccl_gemm_args* g, int splits, int per_sm, cudaStream
     attr_set = true;
   }
   const SkinnyArgs p{reinterpret_cast<__nv_bfloat16*>(g->c), g->m, g->swiglu ? g->n / 2 : g->n, g->k, g->ldc, g->swiglu,
-                     reinterpret_cast<uint32_t*>(g->status)};
+                     reinterpret_cast<uint32_t*>(g->status), timeout_ns};
   const int tiles = (g->n + CG * kSkinnyRows - 1) / (CG * kSkinnyRows);
   return launch_dependent(gemm_skinny_kernel<TN, CG>, dim3(tiles * splits * CG, (g->m + TN - 1) / TN), kThreads,
                           Cfg::smem(per_sm), stream, splits * CG, mw, ma, p, splits, Cfg::stages(per_sm));
 }
 
 // tn tokens per tile, cg CTAs per tile, K split `splits` ways (cg * splits <= 8)
-static int launch_as(const tccl_gemm_args* g, int tn, int cg, int splits, int per_sm, cudaStream_t stream) {
+static int launch_as(const tccl_gemm_args* g, int tn, int cg, int splits, int per_sm, uint64_t timeout_ns,
+                     cudaStream_t stream) {
   if (cg == 1) {
     switch (tn) {
-      case 16: return launch_tn<16, 1>(g, splits, per_sm, stream);
-      case 32: return launch_tn<32, 1>(g, splits, per_sm, stream);
-      case 64: return launch_tn<64, 1>(g, splits, per_sm, stream);
-      default: return launch_tn<128, 1>(g, splits, per_sm, stream);
+      case 16: return launch_tn<16, 1>(g, splits, per_sm, timeout_ns, stream);
+      case 32: return launch_tn<32, 1>(g, splits, per_sm, timeout_ns, stream);
+      case 64: return launch_tn<64, 1>(g, splits, per_sm, timeout_ns, stream);
+      default: return launch_tn<128, 1>(g, splits, per_sm, timeout_ns, stream);
     }
   }
   switch (tn) {
-    case 32: return launch_tn<32, 2>(g, splits, per_sm, stream);
-    case 64: return launch_tn<64, 2>(g, splits, per_sm, stream);
-    case 128: return launch_tn<128, 2>(g, splits, per_sm, stream);
-    default: return launch_tn<256, 2>(g, splits, per_sm, stream);
+    case 32: return launch_tn<32, 2>(g, splits, per_sm, timeout_ns, stream);
+    case 64: return launch_tn<64, 2>(g, splits, per_sm, timeout_ns, stream);
+    case 128: return launch_tn<128, 2>(g, splits, per_sm, timeout_ns, stream);
+    default: return launch_tn<256, 2>(g, splits, per_sm, timeout_ns, stream);
   }
 }
 
@@ -358,7 +359,7 @@ static SkinnyChoice choose(int m, int n, int k) {
   return best;
 }
 
-bool launch_gemm_skinny(const tccl_gemm_args* g, cudaStream_t stream, int* rc) {
+bool launch_gemm_skinny(const tccl_gemm_args* g, cudaStream_t stream, uint64_t timeout_ns, int* rc) {
   if ((long long)g->m * g->n > 6144ll * 6144) return false;  // far beyond where a tile per CTA can win
   // a program multiplies a few shapes over and over: remember their choices (per thread, so without a lock)
   struct Entry { int m, n, k; SkinnyChoice c; };
@@ -366,7 +367,7 @@ bool launch_gemm_skinny(const tccl_gemm_args* g, cudaStream_t stream, int* rc) {
   Entry& e = memo[((unsigned)g->m * 31u + (unsigned)g->n * 17u + (unsigned)g->k) % 64u];
   if (e.m != g->m || e.n != g->n || e.k != g->k) e = Entry{g->m, g->n, g->k, choose(g->m, g->n, g->k)};
   if (!e.c.tn) return false;
-  *rc = launch_as(g, e.c.tn, e.c.cg, e.c.splits, e.c.per_sm, stream);
+  *rc = launch_as(g, e.c.tn, e.c.cg, e.c.splits, e.c.per_sm, timeout_ns, stream);
   return true;
 }
 
