@@ -32,7 +32,7 @@ int tccl_sizeof(const char* name) {
 #define TCCL_SZ(T) if (!strcmp(name, #T)) return (int)sizeof(T);
   TCCL_SZ(tccl_comm) TCCL_SZ(tccl_coll_args) TCCL_SZ(tccl_launch) TCCL_SZ(tccl_barrier_args) TCCL_SZ(tccl_pads_args)
   TCCL_SZ(tccl_tree_args) TCCL_SZ(tccl_arn_args) TCCL_SZ(tccl_gemm_args) TCCL_SZ(tccl_gemm_rs_args)
-  TCCL_SZ(tccl_ag_gemm_args)
+  TCCL_SZ(tccl_ag_gemm_args) TCCL_SZ(tccl_few_rows)
 #undef TCCL_SZ
   return -1;
 }

@@ -58,12 +58,17 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
   run_mainloop2(shp, pol, status ? &fake : nullptr, timeout_ns, trace ? trace + (size_t)blockIdx.x * 64 : nullptr);
 }
 
-int launch_gemm_pair(const tccl_gemm_args* g, int grid, cudaStream_t stream, uint64_t timeout_ns, uint64_t* trace) {
+int check_gemm_args(const tccl_gemm_args* g) {
   if (!g || g->m <= 0 || g->n <= 0 || g->k <= 0) return -TCCL_EINVAL;
   if ((g->lda % 8) || (g->ldb % 8) || (g->ldc % 8) || (g->n % 8) || (g->k % 8)) return -TCCL_EALIGN;
   if (((uintptr_t)g->a | (uintptr_t)g->bt | (uintptr_t)g->c) & 15) return -TCCL_EALIGN;
   if (g->swiglu && (g->n % BN2)) return -TCCL_ESIZE;  // whole gate|up tiles only
-  int rc = 0;
+  return 0;
+}
+
+int launch_gemm_pair(const tccl_gemm_args* g, int grid, cudaStream_t stream, uint64_t timeout_ns, uint64_t* trace) {
+  int rc = check_gemm_args(g);
+  if (rc) return rc;
   if (grid <= 0 && !trace && launch_gemm_skinny(g, stream, timeout_ns, &rc)) return rc;
   CUtensorMap ma, mb128, mb64;
   rc = make_tmap_bf16_kmajor(&ma, g->a, g->m, g->k, g->lda, 128);  // each CTA loads 128 rows of A ...

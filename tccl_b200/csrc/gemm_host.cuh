@@ -80,6 +80,7 @@ namespace gemm2 {
 // gemm_skinny.cu: takes the product (and returns true, with the launch's status in *rc) where one tile per CTA beats
 // the persistent pair kernel: few rows, or fewer tiles than the GPU has pairs of SMs.
 bool launch_gemm_skinny(const tccl_gemm_args* g, cudaStream_t stream, uint64_t timeout_ns, int* rc);
+int check_gemm_args(const tccl_gemm_args* g);  // 0, or what is wrong with the shapes, strides and addresses
 // gemm2.cu: C = A * Bt^T on CTA pairs; grid <= 0: one CTA per SM, and the kernel that suits the shape
 int launch_gemm_pair(const tccl_gemm_args* g, int grid, cudaStream_t stream, uint64_t timeout_ns, uint64_t* trace);
 }  // namespace gemm2

@@ -293,22 +293,25 @@ static int launch_tn(const tccl_gemm_args* g, int splits, int per_sm, uint64_t t
                           Cfg::smem(per_sm), stream, splits * CG, mw, ma, p, splits, Cfg::stages(per_sm));
 }
 
-// tn tokens per tile, cg CTAs per tile, K split `splits` ways (cg * splits <= 8)
+// The tiles there are: `tn` tokens by `cg` * 128 rows of Bt
+static const struct { int tn, cg; } kTiles[] = {{16, 1}, {32, 1}, {64, 1}, {128, 1}, {32, 2}, {64, 2}, {128, 2}, {256, 2}};
+static int max_per_sm(int tn) { return tn <= 128 ? 2 : 1; }
+
+// K split `splits` ways, `per_sm` CTAs on an SM; every split has at least one k-block
 static int launch_as(const tccl_gemm_args* g, int tn, int cg, int splits, int per_sm, uint64_t timeout_ns,
                      cudaStream_t stream) {
-  if (cg == 1) {
-    switch (tn) {
-      case 16: return launch_tn<16, 1>(g, splits, per_sm, timeout_ns, stream);
-      case 32: return launch_tn<32, 1>(g, splits, per_sm, timeout_ns, stream);
-      case 64: return launch_tn<64, 1>(g, splits, per_sm, timeout_ns, stream);
-      default: return launch_tn<128, 1>(g, splits, per_sm, timeout_ns, stream);
-    }
-  }
-  switch (tn) {
-    case 32: return launch_tn<32, 2>(g, splits, per_sm, timeout_ns, stream);
-    case 64: return launch_tn<64, 2>(g, splits, per_sm, timeout_ns, stream);
-    case 128: return launch_tn<128, 2>(g, splits, per_sm, timeout_ns, stream);
-    default: return launch_tn<256, 2>(g, splits, per_sm, timeout_ns, stream);
+  if (splits < 1 || (splits & (splits - 1)) || cg * splits > 8 || splits > (g->k + 63) / 64) return -TCCL_ESIZE;
+  if (per_sm < 1 || per_sm > max_per_sm(tn)) return -TCCL_ESIZE;
+  switch (tn * 4 + cg) {
+    case 16 * 4 + 1: return launch_tn<16, 1>(g, splits, per_sm, timeout_ns, stream);
+    case 32 * 4 + 1: return launch_tn<32, 1>(g, splits, per_sm, timeout_ns, stream);
+    case 64 * 4 + 1: return launch_tn<64, 1>(g, splits, per_sm, timeout_ns, stream);
+    case 128 * 4 + 1: return launch_tn<128, 1>(g, splits, per_sm, timeout_ns, stream);
+    case 32 * 4 + 2: return launch_tn<32, 2>(g, splits, per_sm, timeout_ns, stream);
+    case 64 * 4 + 2: return launch_tn<64, 2>(g, splits, per_sm, timeout_ns, stream);
+    case 128 * 4 + 2: return launch_tn<128, 2>(g, splits, per_sm, timeout_ns, stream);
+    case 256 * 4 + 2: return launch_tn<256, 2>(g, splits, per_sm, timeout_ns, stream);
+    default: return -TCCL_ESIZE;
   }
 }
 
@@ -347,11 +350,10 @@ static float pair_cost(int m, int n, int k) {
 // tn == 0: the pair kernel
 static SkinnyChoice choose(int m, int n, int k) {
   SkinnyChoice best{0, 0, 0, 0, pair_cost(m, n, k)};
-  static const struct { int tn, cg; } kTiles[] = {{16, 1}, {32, 1}, {64, 1}, {128, 1}, {32, 2}, {64, 2}, {128, 2}, {256, 2}};
   for (const auto& t : kTiles) {
     if (t.tn >= 32 && t.tn >= 4 * m) continue;
     for (int splits = 1; splits * t.cg <= 8 && splits <= (k + 63) / 64; splits *= 2)
-      for (int per_sm = 1; per_sm <= (t.tn <= 128 ? 2 : 1); ++per_sm) {
+      for (int per_sm = 1; per_sm <= max_per_sm(t.tn); ++per_sm) {
         const float us = skinny_cost(m, n, k, t.tn, t.cg, splits, per_sm);
         if (us < best.us) best = SkinnyChoice{t.tn, t.cg, splits, per_sm, us};
       }
@@ -359,8 +361,12 @@ static SkinnyChoice choose(int m, int n, int k) {
   return best;
 }
 
+static bool too_many_tiles(int m, int n) {  // far beyond where a tile per CTA can win
+  return (long long)m * n > 6144ll * 6144;
+}
+
 bool launch_gemm_skinny(const tccl_gemm_args* g, cudaStream_t stream, uint64_t timeout_ns, int* rc) {
-  if ((long long)g->m * g->n > 6144ll * 6144) return false;  // far beyond where a tile per CTA can win
+  if (too_many_tiles(g->m, g->n)) return false;
   // a program multiplies a few shapes over and over: remember their choices (per thread, so without a lock)
   struct Entry { int m, n, k; SkinnyChoice c; };
   static thread_local Entry memo[64] = {};
@@ -373,3 +379,18 @@ bool launch_gemm_skinny(const tccl_gemm_args* g, cudaStream_t stream, uint64_t t
 
 }  // namespace gemm2
 }  // namespace tccl
+
+extern "C" int tccl_gemm_choice(int m, int n, int k, tccl_few_rows* out) {
+  using namespace tccl::gemm2;
+  if (m <= 0 || n <= 0 || k <= 0) return -TCCL_EINVAL;
+  const SkinnyChoice c = too_many_tiles(m, n) ? SkinnyChoice{} : choose(m, n, k);
+  *out = tccl_few_rows{c.tn, c.cg, c.splits, c.per_sm};
+  return 0;
+}
+
+extern "C" int tccl_gemm_few_rows(const tccl_gemm_args* g, const tccl_few_rows* f, void* stream) {
+  using namespace tccl::gemm2;
+  const int rc = check_gemm_args(g);
+  if (rc) return rc;
+  return launch_as(g, f->tokens, f->ctas, f->splits, f->per_sm, 2000000000ull, reinterpret_cast<cudaStream_t>(stream));
+}

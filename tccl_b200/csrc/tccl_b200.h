@@ -264,6 +264,16 @@ int tccl_gemm_bf16(const tccl_gemm_args*, int grid, void* stream);
  * With grid <= 0 products of few rows take a kernel of their own. */
 int tccl_gemm_bf16_pair(const tccl_gemm_args*, int grid, void* stream);
 
+/* A configuration of the kernel for few rows: `tokens` rows of a and `ctas` * 128 rows of bt per tile (ctas 1 or 2: a
+ * pair), k split `splits` ways over a cluster of ctas * splits <= 8, `per_sm` CTAs on an SM. */
+typedef struct tccl_few_rows {
+  int32_t tokens, ctas, splits, per_sm;
+} tccl_few_rows;
+/* what tccl_gemm_bf16_pair takes for a product; tokens == 0: the persistent pair kernel */
+int tccl_gemm_choice(int m, int n, int k, tccl_few_rows* out);
+/* test hook: the same product in a named configuration; -TCCL_ESIZE if there is none such */
+int tccl_gemm_few_rows(const tccl_gemm_args*, const tccl_few_rows*, void* stream);
+
 /* ---- fused GEMM -> reduce-scatter (rows scattered over the ranks) ---------- */
 typedef struct tccl_gemm_rs_args {
   const void* a;   /* this rank's [m, k] activations (its K-slice), k contiguous */

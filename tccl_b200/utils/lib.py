@@ -86,6 +86,10 @@ class GemmArgs(C.Structure):
     ]
 
 
+class FewRows(C.Structure):
+    _fields_ = [("tokens", C.c_int32), ("ctas", C.c_int32), ("splits", C.c_int32), ("per_sm", C.c_int32)]
+
+
 class GemmRsArgs(C.Structure):
     _fields_ = [
         ("a", C.c_uint64), ("bt", C.c_uint64), ("out", C.c_uint64),

@@ -20,7 +20,7 @@ def test_struct_layout_matches_c():
     pairs = {"tccl_comm": L.Comm, "tccl_coll_args": L.CollArgs, "tccl_launch": L.Launch,
              "tccl_barrier_args": L.BarrierArgs, "tccl_pads_args": L.PadsArgs, "tccl_tree_args": L.TreeArgs,
              "tccl_arn_args": L.ArnArgs, "tccl_gemm_args": L.GemmArgs, "tccl_gemm_rs_args": L.GemmRsArgs,
-             "tccl_ag_gemm_args": L.AgGemmArgs}
+             "tccl_ag_gemm_args": L.AgGemmArgs, "tccl_few_rows": L.FewRows}
     for name, mirror in pairs.items():
         assert lib.tccl_sizeof(name.encode()) == C.sizeof(mirror), name
     assert lib.tccl_sizeof(b"no_such_struct") == -1
