@@ -509,3 +509,34 @@ def test_large_all_reduce_into_ordinary_memory_uses_the_staged_two_shot(emu_worl
     for r in range(W):
         assert_close_to_sum(out[r], ref, torch.bfloat16, W)
         assert torch.equal(out2[r], out[r]) and torch.equal(x[r], keep[r])
+
+
+@pytest.mark.parametrize("W", [5, 6, 7])
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("per", [8, 8 * 4096 + 8])
+def test_flat_collectives_of_odd_worlds(emu_worlds, W, dtype, per):
+    """World sizes with kernel instances of their own, and those that share the run-time one."""
+    import tccl_b200 as tccl
+
+    w = emu_worlds(W)
+    n = per * W
+    x = make_inputs(w, W, n, dtype, 7000 + W)
+    ref = ref_sum(x)
+    out = w.empty(n, dtype)
+    for algo in ["oneshot_p2p", "twoshot_p2p", "twoshot_pipe_p2p"] + (["push_p2p"] if n * 4 <= w.push_max_bytes() else []):
+        for p in out.parts:
+            p.fill_(77.0)
+        tccl.all_reduce(x, out=out, algo=algo, world=w)
+        torch.cuda.synchronize()
+        w.check()
+        for r in range(W):
+            assert_close_to_sum(out[r], ref, dtype, W)
+    shares = tccl.reduce_scatter(x, world=w)
+    pulled = tccl.all_gather(x, algo="pull", world=w)
+    pushed = tccl.all_gather(x, out=w.empty((W, n), dtype), algo="push", world=w)
+    torch.cuda.synchronize()
+    w.check()
+    rows = torch.stack(list(x.parts))
+    for r in range(W):
+        assert_close_to_sum(shares[r], ref[r * per: (r + 1) * per], dtype, W)
+        assert torch.equal(pulled[r], rows) and torch.equal(pushed[r], rows)

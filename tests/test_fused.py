@@ -184,3 +184,39 @@ def test_tensor_parallel_mlp_matches_unsharded_fp32(emu_worlds, W):
     got = torch.cat([o.float() for o in outs])
     err = (got - ref).abs()
     assert bool((err <= ref.abs() * 2 ** -6 + 3e-3).all()), err.max().item()
+
+
+@pytest.mark.parametrize("M", [128, 384, 640, 4224])
+@pytest.mark.parametrize("swiglu", [False, True])
+def test_one_rank_rows_short_of_a_pair_tile(emu_worlds, M, swiglu):
+    """One rank takes any multiple of 128 rows: the last 256-row tile of the pair kernels hangs over the end, and nothing
+    is written there."""
+    import tccl_b200 as tccl
+
+    w = emu_worlds(1)
+    N, K = 768, 200
+    a, bt = _rand((M, K), 6000 + M), _rand((N, K), 6100, 0.05)
+    cols = N // 2 if swiglu else N
+    full = torch.full((M + 256, cols), 77.0, dtype=torch.bfloat16, device="cuda")
+    ref = a.float() @ bt.float().t()
+    sums = 1e-3 * (K ** 0.5) * 0.05  # fp32 sums in another order
+    for _ in range(2):
+        outs, a_full = tccl.all_gather_gemm([a], [bt], out=[full[:M]], swiglu=swiglu, world=w)
+        torch.cuda.synchronize()
+        w.check()
+        if swiglu:
+            gr, ur = (t.reshape(M, -1) for t in ref.view(M, -1, 2, 128).unbind(2))
+            want = torch.nn.functional.silu(gr) * ur
+            bound = want.abs() * (2 ** -8 + 1e-5) + sums * (1.1 * ur.abs() + gr.abs() + 1e-3)
+        else:
+            want, bound = ref, ref.abs() * 2 ** -8 + sums
+        err = (outs[0].float() - want).abs()
+        assert bool((err <= bound).all()), f"worst ratio {(err / bound).max().item()}"
+        assert bool((full[M:] == 77.0).all()) and torch.equal(a_full[0], a)
+    if not swiglu:
+        full.fill_(77.0)
+        tccl.gemm_reduce_scatter([a], [bt], out=[full[:M]], world=w)
+        torch.cuda.synchronize()
+        w.check()
+        err = (full[:M].float() - ref).abs()
+        assert bool((err <= ref.abs() * 2 ** -8 + sums).all()) and bool((full[M:] == 77.0).all())
