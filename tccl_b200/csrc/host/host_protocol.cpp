@@ -105,6 +105,7 @@ struct TreeJob {
   uint64_t ring_stride;         // elements per ring slot: fixed for the communicator, >= any chunk
   int parent[2], left[2], right[2], child_slot[2];
   bool pull_down;               // way down: children copy the sum out of their parent's buffer and acknowledge
+  bool early_post;              // see tree_worker
 };
 constexpr int kDepth = TCCL_TREE_RING_DEPTH;
 
@@ -112,8 +113,46 @@ float* ring_slot(const TreeJob& j, int rank, int tree, int cslot, uint32_t seq) 
   return j.ring[rank] + ((size_t)((tree * 2 + cslot) * kDepth) + seq % kDepth) * j.ring_stride;
 }
 
-// one (tree, direction) worker = what one CTA does on the device (K = 1 slice): the push
-// protocol of tree_allreduce.cu with the same counters, running totals and ring reuse rule
+constexpr int kAhead = 4;      // slices between polling and posting, as in tree_allreduce.cu
+constexpr int kDataWarps = 2;
+
+// an mbarrier: an arrival count and a phase
+struct Mbar {
+  std::atomic<int> pending{0};
+  std::atomic<uint32_t> phase{0};
+  int count = 0;
+  void init(int n) {
+    count = n;
+    pending.store(n, std::memory_order_relaxed);
+    phase.store(0, std::memory_order_relaxed);
+  }
+  void arrive() {
+    if (pending.fetch_sub(1, std::memory_order_acq_rel) == 1) {
+      pending.store(count, std::memory_order_relaxed);
+      phase.fetch_add(1, std::memory_order_release);
+    }
+  }
+  // like mbarrier.try_wait.parity in a loop: returns once the phase with this parity has completed
+  void wait(uint32_t parity) const {
+    while ((phase.load(std::memory_order_acquire) & 1u) == parity) std::this_thread::yield();
+  }
+  // bounded form: false once `give_up` says so
+  template <class F> bool wait(uint32_t parity, const F& give_up) const {
+    while ((phase.load(std::memory_order_acquire) & 1u) == parity) {
+      if (give_up()) return false;
+      std::this_thread::yield();
+    }
+    return true;
+  }
+};
+
+// One (tree, direction) worker = what one CTA does on the device (K = 1 slice): the protocol of tree_allreduce.cu with
+// the same counters, running totals and ring reuse rule, and the same split inside the CTA — a polling warp that waits
+// for the counters up to kAhead slices ahead of the data, data warps that only load, add and store, and a posting warp
+// that raises the counters behind them — with the three rings of mbarriers that hand a slice over: `ready` (inputs
+// there, destination free), `done` (every data warp has issued its stores), `sent` (counters raised).
+// `early_post` is a mistake kept so that the sanitizer can be seen to catch it: the posting warp goes by the FIRST data
+// warp that is done with a slice.
 void tree_worker(const HostComm& c, const TreeJob& j, int tree, bool is_up, clk::time_point deadline, const Faults& f) {
   const int me = c.rank, parent = j.parent[tree], left = j.left[tree], right = j.right[tree];
   const int cslot = j.child_slot[tree];
@@ -122,64 +161,104 @@ void tree_worker(const HostComm& c, const TreeJob& j, int tree, bool is_up, clk:
   const int role = (is_up ? 0 : 2) + tree;
   uint32_t* seq_word = c.local + TCCL_LOCAL_TREE_SEQ + role * TCCL_TREE_MAX_CTAS;
   const uint32_t base = *seq_word;
-  if (is_up) {
-    for (uint64_t n = 0; n < mine; ++n) {
-      if (f.stop_after_chunk >= 0 && n >= (uint64_t)f.stop_after_chunk) return;  // injected: this rank stops here
+  uint64_t slices = is_up || parent >= 0 ? mine : 0;  // the root has no way down
+  bool stopped = false;                               // injected: this rank stops here
+  if (f.stop_after_chunk >= 0 && slices > (uint64_t)f.stop_after_chunk) {
+    slices = (uint64_t)f.stop_after_chunk;
+    stopped = true;
+  }
+  Mbar ready[kAhead], done[kAhead], sent[kAhead];
+  for (int i = 0; i < kAhead; ++i) {
+    ready[i].init(1);
+    done[i].init(j.early_post ? 1 : kDataWarps);
+    sent[i].init(1);
+  }
+  std::atomic<int> abort_cta{0};
+  const auto late = deadline + std::chrono::nanoseconds(c.timeout_ns / 4) + std::chrono::milliseconds(1);
+  auto give_up = [&] { return abort_cta.load(std::memory_order_relaxed) != 0 || clk::now() > late; };
+  auto fail = [&] { abort_cta.store(1, std::memory_order_relaxed); };
+
+  auto post = [&] {
+    for (uint64_t n = 0; n < slices; ++n) {
       const uint32_t g = base + (uint32_t)n;
-      if (left >= 0 && !wait_reach(up_flag(c, me, tree, 0, 0), g + 1u, c, deadline, tree, left, TCCL_W_TREE_UP)) return;
-      if (right >= 0 && !wait_reach(up_flag(c, me, tree, 0, 1), g + 1u, c, deadline, tree, right, TCCL_W_TREE_UP)) return;
-      if (parent >= 0 &&
-          !wait_reach(ack_flag(c, me, tree, 0), g + 1u - (uint32_t)kDepth, c, deadline, tree, parent, TCCL_W_TREE_UP))
-        return;
-      const uint64_t lo = (2 * n + tree) * j.chunk, hi = std::min(lo + j.chunk, j.numel);
-      const float* lr = left >= 0 ? ring_slot(j, me, tree, 0, g) : nullptr;
-      const float* rr = right >= 0 ? ring_slot(j, me, tree, 1, g) : nullptr;
-      float* pr = parent >= 0 ? ring_slot(j, parent, tree, cslot, g) : nullptr;
-      for (uint64_t i = lo; i < hi; ++i) {
-        const float v = j.in[i] + (lr ? lr[i - lo] : 0.f) + (rr ? rr[i - lo] : 0.f);
-        if (pr) {
-          pr[i - lo] = v;
-        } else {  // the root: the final value goes to its own and its children's result buffers
-          j.buf[me][i] = v;
-          if (!j.pull_down) {
-            if (left >= 0) j.buf[left][i] = v;
-            if (right >= 0) j.buf[right][i] = v;
-          }
-        }
-      }
-      if (parent >= 0) {
+      if (!done[n % kAhead].wait((uint32_t)(n / kAhead) & 1u, give_up)) return fail();
+      if (is_up && parent >= 0) {
         A(up_flag(c, parent, tree, 0, cslot)).store(g + 1u, std::memory_order_release);
       } else {
         if (left >= 0) A(down_flag(c, left, tree, 0)).store(g + 1u, std::memory_order_release);
         if (right >= 0) A(down_flag(c, right, tree, 0)).store(g + 1u, std::memory_order_release);
       }
-      if (left >= 0) A(ack_flag(c, left, tree, 0)).store(g + 1u, std::memory_order_release);
-      if (right >= 0) A(ack_flag(c, right, tree, 0)).store(g + 1u, std::memory_order_release);
-    }
-  } else {
-    for (uint64_t n = 0; parent >= 0 && n < mine; ++n) {
-      if (f.stop_after_chunk >= 0 && n >= (uint64_t)f.stop_after_chunk) return;
-      const uint32_t g = base + (uint32_t)n;
-      if (!wait_reach(down_flag(c, me, tree, 0), g + 1u, c, deadline, 2 + tree, parent, TCCL_W_TREE_DOWN)) return;
-      const uint64_t lo = (2 * n + tree) * j.chunk, hi = std::min(lo + j.chunk, j.numel);
-      if (j.pull_down) {
-        std::memcpy(j.buf[me] + lo, j.buf[parent] + lo, (hi - lo) * sizeof(float));
+      if (is_up) {
+        if (left >= 0) A(ack_flag(c, left, tree, 0)).store(g + 1u, std::memory_order_release);
+        if (right >= 0) A(ack_flag(c, right, tree, 0)).store(g + 1u, std::memory_order_release);
+      } else if (j.pull_down) {  // this slice of the parent's buffer is no longer needed
         A(dack_flag(c, parent, tree, 0, cslot)).store(g + 1u, std::memory_order_release);
+      }
+      sent[n % kAhead].arrive();
+    }
+  };
+  auto poll = [&] {
+    for (uint64_t n = 0; n < slices; ++n) {
+      const uint32_t g = base + (uint32_t)n;
+      if (n >= (uint64_t)kAhead && !sent[n % kAhead].wait((uint32_t)(n / kAhead - 1) & 1u, give_up)) return fail();
+      if (is_up) {
+        // the children's partials are in my ring; the slot to be filled at the parent is free
+        if (left >= 0 && !wait_reach(up_flag(c, me, tree, 0, 0), g + 1u, c, deadline, tree, left, TCCL_W_TREE_UP)) return fail();
+        if (right >= 0 && !wait_reach(up_flag(c, me, tree, 0, 1), g + 1u, c, deadline, tree, right, TCCL_W_TREE_UP)) return fail();
+        if (parent >= 0 &&
+            !wait_reach(ack_flag(c, me, tree, 0), g + 1u - (uint32_t)kDepth, c, deadline, tree, parent, TCCL_W_TREE_UP))
+          return fail();
+      } else if (!wait_reach(down_flag(c, me, tree, 0), g + 1u, c, deadline, 2 + tree, parent, TCCL_W_TREE_DOWN)) {
+        return fail();
+      }
+      ready[n % kAhead].arrive();
+    }
+    if (j.pull_down && !is_up && mine && !stopped) {
+      // the caller may overwrite this rank's buffer once the call returns: wait until the children have copied it
+      const uint32_t want = base + (uint32_t)mine;
+      if (left >= 0 && !wait_reach(dack_flag(c, me, tree, 0, 0), want, c, deadline, 2 + tree, left, TCCL_W_TREE_DOWN)) return fail();
+      if (right >= 0 && !wait_reach(dack_flag(c, me, tree, 0, 1), want, c, deadline, 2 + tree, right, TCCL_W_TREE_DOWN)) return fail();
+    }
+  };
+  auto data = [&](int warp) {
+    for (uint64_t n = 0; n < slices; ++n) {
+      const uint32_t g = base + (uint32_t)n;
+      if (!ready[n % kAhead].wait((uint32_t)(n / kAhead) & 1u, give_up)) return fail();
+      const uint64_t clo = (2 * n + tree) * j.chunk, chi = std::min(clo + j.chunk, j.numel);
+      const uint64_t per = (chi - clo + kDataWarps - 1) / kDataWarps;  // the warps share the slice
+      const uint64_t lo = std::min(clo + per * warp, chi), hi = std::min(lo + per, chi);
+      if (is_up) {
+        const float* lr = left >= 0 ? ring_slot(j, me, tree, 0, g) : nullptr;
+        const float* rr = right >= 0 ? ring_slot(j, me, tree, 1, g) : nullptr;
+        float* pr = parent >= 0 ? ring_slot(j, parent, tree, cslot, g) : nullptr;
+        for (uint64_t i = lo; i < hi; ++i) {
+          const float v = j.in[i] + (lr ? lr[i - clo] : 0.f) + (rr ? rr[i - clo] : 0.f);
+          if (pr) {
+            pr[i - clo] = v;
+          } else {  // the root: the final value goes to its own and its children's result buffers
+            j.buf[me][i] = v;
+            if (!j.pull_down) {
+              if (left >= 0) j.buf[left][i] = v;
+              if (right >= 0) j.buf[right][i] = v;
+            }
+          }
+        }
+      } else if (j.pull_down) {
+        std::memcpy(j.buf[me] + lo, j.buf[parent] + lo, (hi - lo) * sizeof(float));
       } else {
         if (left >= 0) std::memcpy(j.buf[left] + lo, j.buf[me] + lo, (hi - lo) * sizeof(float));
         if (right >= 0) std::memcpy(j.buf[right] + lo, j.buf[me] + lo, (hi - lo) * sizeof(float));
       }
-      if (left >= 0) A(down_flag(c, left, tree, 0)).store(g + 1u, std::memory_order_release);
-      if (right >= 0) A(down_flag(c, right, tree, 0)).store(g + 1u, std::memory_order_release);
+      if (j.early_post && warp) continue;
+      done[n % kAhead].arrive();
     }
-    if (j.pull_down && mine) {
-      // the caller may overwrite this rank's buffer once the call returns: wait until the children have copied it
-      const uint32_t want = base + (uint32_t)mine;
-      if (left >= 0 && !wait_reach(dack_flag(c, me, tree, 0, 0), want, c, deadline, 2 + tree, left, TCCL_W_TREE_DOWN)) return;
-      if (right >= 0 && !wait_reach(dack_flag(c, me, tree, 0, 1), want, c, deadline, 2 + tree, right, TCCL_W_TREE_DOWN)) return;
-    }
-  }
-  *seq_word = base + (uint32_t)mine;
+  };
+  std::vector<std::thread> th;
+  th.emplace_back(post);
+  th.emplace_back(poll);
+  for (int w = 0; w < kDataWarps; ++w) th.emplace_back(data, w);
+  for (auto& x : th) x.join();
+  if (!stopped && !abort_cta.load()) *seq_word = base + (uint32_t)mine;
 }
 
 }  // namespace
@@ -201,7 +280,8 @@ struct hp_tree {
   uint64_t ring[TCCL_MAX_WORLD];  // 4 * TCCL_TREE_RING_DEPTH * ring_stride floats per rank
   uint64_t numel, chunk, ring_stride;
   int32_t parent[2], left[2], right[2], child_slot[2];
-  int32_t pull_down, pad_;        // 1: children copy the sum out of their parent's buffer (the large-message form)
+  int32_t pull_down;              // 1: children copy the sum out of their parent's buffer (the large-message form)
+  int32_t early_post;             // 1: the mistake that tree_worker keeps
 };
 
 static HostComm to_comm(const hp_comm* h) {
@@ -239,6 +319,7 @@ int hp_tree_allreduce(const hp_comm* h, const hp_tree* t, const hp_faults* f) {
   j.chunk = t->chunk;
   j.ring_stride = t->ring_stride;
   j.pull_down = t->pull_down != 0;
+  j.early_post = t->early_post != 0;
   if (j.chunk > j.ring_stride) return 0;
   for (int i = 0; i < 2; ++i) {
     j.parent[i] = t->parent[i];
@@ -262,7 +343,7 @@ int hp_tree_allreduce(const hp_comm* h, const hp_tree* t, const hp_faults* f) {
 // -fsanitize=thread this checks that every plain (non-atomic) access of the data
 // buffers is ordered by the release/acquire flag protocol — the race detector the
 // GPU side cannot have.  Returns 0 on success, a positive code otherwise.
-extern "C" int hp_selftest_threads(int world, int numel, int chunk, int rounds) {
+static int tree_selftest(int world, int numel, int chunk, int rounds, bool early_post) {
   if (world < 1 || world > TCCL_MAX_WORLD) return 100;
   constexpr int kCalls = 6;  // back to back, no barrier in between, alternating chunk sizes and forms of the way down
   std::vector<std::vector<uint32_t>> flags(world, std::vector<uint32_t>(TCCL_FLAG_WORDS, 0u));
@@ -310,7 +391,7 @@ extern "C" int hp_selftest_threads(int world, int numel, int chunk, int rounds) 
       h.rank = r;
       for (int p = 0; p < world; ++p) h.flags[p] = reinterpret_cast<uint64_t>(flags[p].data());
       h.local = reinterpret_cast<uint64_t>(local[r].data());
-      h.timeout_ns = 20ull * 1000 * 1000 * 1000;
+      h.timeout_ns = (early_post ? 1ull : 20ull) * 1000 * 1000 * 1000;  // the mistake may also end in a wait that runs out
       hp_faults none{-1, 0, -1};
       int ok = hp_barrier(&h, 1, rounds, &none);
       for (int call = 0; call < kCalls && ok; ++call) {
@@ -326,6 +407,7 @@ extern "C" int hp_selftest_threads(int world, int numel, int chunk, int rounds) 
         t.numel = (uint64_t)numel;
         t.chunk = (uint64_t)((call & 1) ? std::max(1, chunk / 2) : chunk);
         t.ring_stride = (uint64_t)chunk;
+        t.early_post = early_post;
         t.pull_down = (call >> 1) & 1;  // push, push, pull, pull: both forms and the change between them
         for (int tr = 0; tr < 2; ++tr) {
           int parent, left, right;
@@ -352,6 +434,13 @@ extern "C" int hp_selftest_threads(int world, int numel, int chunk, int rounds) 
   for (int r = 0; r < world; ++r)
     if (!results[r]) return 1;
   return bad.load();
+}
+extern "C" int hp_selftest_threads(int world, int numel, int chunk, int rounds) {
+  return tree_selftest(world, numel, chunk, rounds, false);
+}
+// the posting warp of every CTA goes by the first data warp that is done: must be caught
+extern "C" int hp_selftest_tree_early_post(int world, int numel, int chunk) {
+  return tree_selftest(world, numel, chunk, 1, true);
 }
 
 // ---------------------------------------------------------------------------
@@ -630,26 +719,6 @@ extern "C" int hp_selftest_push(int world, int calls, int scheme) {
 // released or refilled too early shows up as a data race.  Ranks meet at the epoch barrier on
 // entry and on exit; two calls run back to back, in place.
 namespace {
-struct Mbar {
-  std::atomic<int> pending{0};
-  std::atomic<uint32_t> phase{0};
-  int count = 0;
-  void init(int n) {
-    count = n;
-    pending.store(n, std::memory_order_relaxed);
-    phase.store(0, std::memory_order_relaxed);
-  }
-  void arrive() {
-    if (pending.fetch_sub(1, std::memory_order_acq_rel) == 1) {
-      pending.store(count, std::memory_order_relaxed);
-      phase.fetch_add(1, std::memory_order_release);
-    }
-  }
-  // like mbarrier.try_wait.parity in a loop: returns once the phase with this parity has completed
-  void wait(uint32_t parity) const {
-    while ((phase.load(std::memory_order_acquire) & 1u) == parity) std::this_thread::yield();
-  }
-};
 struct CopyJob {
   float* dst;
   const float* src;

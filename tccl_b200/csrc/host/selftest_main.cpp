@@ -5,6 +5,7 @@
 #include <cstring>
 
 extern "C" int hp_selftest_threads(int world, int numel, int chunk, int rounds);
+extern "C" int hp_selftest_tree_early_post(int world, int numel, int chunk);
 extern "C" int hp_selftest_gemm_rs(int world, int ctas, int tiles_per_owner, int calls);
 extern "C" int hp_selftest_ag(int world, int movers, int consumers, int row_tiles, int calls);
 extern "C" int hp_selftest_push(int world, int calls, int scheme);
@@ -37,6 +38,12 @@ int main(int argc, char** argv) {
     // output stages freed when their copies are issued, not when they have been read: expected to be reported
     const int rc = hp_selftest_bulk(std::atoi(argv[2]), 2, 4096, 12, 2, 1);
     std::printf("hp_selftest_bulk(broken variant) -> %d\n", rc);
+    return rc;
+  }
+  if (argc > 2 && std::strcmp(argv[1], "tree-broken-variant") == 0) {
+    // counters raised when one of a CTA's data warps is done with a slice: expected to be reported
+    const int rc = hp_selftest_tree_early_post(std::atoi(argv[2]), 1 << 13, 1 << 8);
+    std::printf("hp_selftest_tree_early_post -> %d\n", rc);
     return rc;
   }
   if (argc > 2 && std::strcmp(argv[1], "pair-exit-broken-variant") == 0) {

@@ -27,7 +27,7 @@ class HpTree(C.Structure):
     _fields_ = [("inp", C.c_uint64), ("buf", C.c_uint64 * MAXW), ("ring", C.c_uint64 * MAXW),
                 ("numel", C.c_uint64), ("chunk", C.c_uint64), ("ring_stride", C.c_uint64),
                 ("parent", C.c_int32 * 2), ("left", C.c_int32 * 2), ("right", C.c_int32 * 2),
-                ("child_slot", C.c_int32 * 2), ("pull_down", C.c_int32), ("pad_", C.c_int32)]
+                ("child_slot", C.c_int32 * 2), ("pull_down", C.c_int32), ("early_post", C.c_int32)]
 
 
 def _lib(path: Optional[str] = None) -> C.CDLL:

@@ -73,7 +73,7 @@ def test_rank_that_stops_mid_all_reduce(pull_down):
 def test_protocol_is_race_free_under_thread_sanitizer(W):
     """Ranks (and CTAs) as threads of one process, instrumented with ThreadSanitizer: every plain
     access of the data buffers must be ordered by the release/acquire flags.  Covers the barrier,
-    the double-tree pipeline (pushed and pulled way down), the flag-in-line tree (slot depth 4 and 1),
+    the double-tree pipeline (pushed and pulled way down; polling, data and posting warps of a CTA), the flag-in-line tree (slot depth 4 and 1),
     the GEMM -> reduce-scatter tile flags
     (deferred release, final phase, epoch hand-over across calls), the all-gather -> GEMM arrival
     flags, the push all-reduce with changing sizes and grids, the barrier-free CTA-pair forms of both
@@ -183,5 +183,22 @@ def test_a_cta_pair_that_leaves_before_its_last_arrivals_have_landed_is_caught(t
     except RuntimeError as e:
         pytest.skip(str(e)[:200])
     r = subprocess.run([str(exe), "pair-exit-broken-variant", str(tiles)], capture_output=True, text=True, timeout=300)
+    out = r.stdout + r.stderr
+    assert "ThreadSanitizer: data race" in out or r.returncode != 0, out[-2000:]
+
+
+def test_thread_sanitizer_flags_counters_raised_before_every_data_warp_is_done():
+    """Inside a CTA of the chunked tree the data warps hand a slice to the posting warp through an mbarrier that counts
+    ALL of them; a posting warp that goes by the first one lets the parent read a slice that is still being written.
+    The hand-over that the kernel uses runs clean in test_protocol_is_race_free_under_thread_sanitizer."""
+    import subprocess
+
+    from tccl_b200.utils import build as B
+
+    try:
+        exe = B.build_host_tsan()
+    except RuntimeError as e:
+        pytest.skip(str(e)[:200])
+    r = subprocess.run([str(exe), "tree-broken-variant", "4"], capture_output=True, text=True, timeout=300)
     out = r.stdout + r.stderr
     assert "ThreadSanitizer: data race" in out or r.returncode != 0, out[-2000:]
