@@ -54,6 +54,7 @@ struct alignas(64) AgGemmPairParams {
 };
 
 struct AgGemmPairPolicy {
+  static constexpr bool kEpiBarrier = false;
   const tccl_comm* c;
   const AgGemmPairParams* p;
   int pair, npairs;

@@ -10,6 +10,7 @@ namespace tccl {
 namespace gemm {
 
 struct PlainPolicy {
+  static constexpr bool kEpiBarrier = false;
   const CUtensorMap* map_a;
   __nv_bfloat16* C;
   int M, N, ldc;

@@ -8,6 +8,7 @@ namespace tccl {
 namespace gemm2 {
 
 struct PlainPolicy2 {
+  static constexpr bool kEpiBarrier = false;
   const CUtensorMap *map_a, *map_b128, *map_b64;
   __nv_bfloat16* C;
   int M, N, ldc;  // N: rows of Bt

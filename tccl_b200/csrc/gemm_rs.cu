@@ -44,6 +44,7 @@ struct alignas(64) GemmRsParams {
 __device__ __forceinline__ void epi_bar() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
 
 struct GemmRsPolicy {
+  static constexpr bool kEpiBarrier = true;
   const tccl_comm* c;
   const GemmRsParams* p;
   int bid, nb;
@@ -125,8 +126,7 @@ struct GemmRsPolicy {
         bulk_wait_read<0>();  // both chunks are free for the next tile
         pending_flag = c->flags[owner] + TCCL_FLAG_TILE + me * TCCL_MAX_TILES + lt;
       }
-      epi_bar();
-      return !*ab.flag;
+      return agree<true>(!*ab.flag);
     }
   }
 };

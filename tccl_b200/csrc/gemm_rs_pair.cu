@@ -58,6 +58,7 @@ struct alignas(64) GemmRsPairParams {
 __device__ __forceinline__ void epi_bar2() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
 
 struct GemmRsPairPolicy {
+  static constexpr bool kEpiBarrier = true;
   const tccl_comm* c;
   const GemmRsPairParams* p;
   int pair, npairs;
@@ -205,8 +206,7 @@ struct GemmRsPairPolicy {
       bulk_wait_read<0>();
       pending_flag = c->flags[owner] + TCCL_FLAG_TILE + me * TCCL_MAX_TILES + lt;
     }
-    epi_bar2();
-    return !*ab.flag;
+    return agree<true>(!*ab.flag);
   }
   // the copy engine has the tile and the accumulator is free again: use the wait for reduction work
   __device__ __forceinline__ void between_tiles(int quad, int lane, const Abort&) { try_reduce(quad, lane, 2); }

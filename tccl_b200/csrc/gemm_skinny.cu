@@ -226,7 +226,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     // read the same quarter of the tensor memory's lanes; they share its columns.
     const int quad = warp & 3, row = quad * 32 + lane;
     float* part = reinterpret_cast<float*>(base);
-    if (mbar_wait(done, 0, ab)) {
+    if (agree<false>(mbar_wait(done, 0, ab))) {
       tc_fence_after();
       const uint32_t taddr = tmem + ((uint32_t)(quad * 32) << 16);
 #pragma unroll 1

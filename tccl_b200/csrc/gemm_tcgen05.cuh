@@ -174,6 +174,20 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, const 
   return true;
 }
 
+// One verdict on a wait for the threads that go on to something they do together: a warp-wide instruction, or (kCta) a
+// named barrier of the four epilogue warps.  Every lane polls by itself, and while a wait is being given up one may see
+// that just before the phase completes and another just after; without a vote the two would then wait for each other at
+// different places for good, which no time limit covers.
+template <bool kCta>
+__device__ __forceinline__ bool agree(bool ok) {
+  if (!kCta) return __all_sync(0xffffffffu, ok);
+  uint32_t all;
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %1, 0;\n\tbar.red.and.pred q, 1, 128, p;\n\tselp.u32 %0, 1, 0, q;\n\t}"
+      : "=r"(all) : "r"((uint32_t)ok) : "memory");
+  return all != 0;
+}
+
 // ------------------------------------------------------------------ mainloop
 struct Shape {
   int M, N, K;
@@ -210,6 +224,7 @@ struct SmemLayout {
 // A schedule maps the i-th tile of this CTA to (m_tile, n_tile); hooks:
 //   Policy::tile(i, m_tile, n_tile)          -> false when the CTA is out of tiles
 //   Policy::a_tile(m_tile, map, y)           -> which tensor map / row coordinate holds the A rows
+//   Policy::kEpiBarrier                      -> the epilogue meets at named barrier 1 (128 threads)
 //   Policy::before_load(m_tile, n_tile, ab)  -> runs in the producer thread before the
 //                                               tile's first TMA load (wait for remote rows)
 //   Policy::epilogue(m_tile, n_tile, acc_taddr, quad, lane, ab, sm)
@@ -318,7 +333,7 @@ __device__ void run_mainloop(const CUtensorMap* map_b, const Shape shp, Policy& 
     int mt, nt;
     for (int i = 0; ok && pol.tile(i, mt, nt); ++i) {
       const int acc = i & 1;
-      ok = mbar_wait(sm.tmem_full + acc, (i >> 1) & 1, ab);
+      ok = agree<Policy::kEpiBarrier>(mbar_wait(sm.tmem_full + acc, (i >> 1) & 1, ab));
       if (!ok) break;
       tc_fence_after();
       const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + acc * BN;

@@ -252,6 +252,7 @@ __device__ __forceinline__ void store_rows_swiglu(uint8_t* buf, __nv_bfloat16* C
 //   b_tile(nt, half, cta, map, y)          -> tensor map of Bt (box of 128 rows for half == 0, of 64 rows else) and
 //                                             the first Bt row CTA `cta` of the pair loads; b_rows_default() below
 //                                             is the plain layout (the pair's rows are consecutive)
+//   kEpiBarrier                            -> epilogue or between_tiles meets at named barrier 1 (128 threads)
 //   before_load(mt, nt, ab)                -> producer thread, before the CTA's first load of its m tile
 //   epilogue(mt, nt, col0, ncols, taddr, quad, lane, ab, sm)
 //                                          -> 4 epilogue warps of each CTA; columns [col0, col0 + ncols) of
@@ -393,7 +394,7 @@ __device__ void run_mainloop2(const Shape shp, Policy& pol, const tccl_comm* com
     for (int i = 0; ok && pol.tile(i, mt, nt, half); ++i) {
       mt += (int)cta;
       const int acc = i & 1;
-      ok = mbar_wait(sm.tmem_full + acc, (i >> 1) & 1, ab);
+      ok = agree<Policy::kEpiBarrier>(mbar_wait(sm.tmem_full + acc, (i >> 1) & 1, ab));
       if (!ok) break;
       tc_fence_after();
       const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + acc * BN2;

@@ -1311,3 +1311,47 @@ extern "C" int hp_selftest_pair_exit(int tiles, int rounds, int drain) {
   wire.join();
   return net.strays.load() ? 1 : 0;
 }
+
+// ---------------------------------------------------------------------------
+// Model of a wait whose lanes go on to something they do together (`agree` in gemm_tcgen05.cuh: the data warps of
+// tree_allreduce.cu, the epilogue warps of the GEMMs).  Every lane polls the mbarrier by itself, and while the wait is being given up elsewhere in the CTA one lane may see that just before the phase completes and the
+// others just after: here lane 0 looks first.  `uniform` = 1 (the kernel): the lanes vote and leave or go on together.
+// `uniform` = 0 is the mistake, kept to show that it is caught: the lanes that go on wait for lane 0 at their next
+// __syncwarp or named barrier, lane 0 waits for them at the CTA's last __syncthreads, and the CTA never returns.  Returns 1 where a
+// barrier of the model is still short of a lane after a second.
+extern "C" int hp_selftest_warp_verdict(int uniform) {
+  constexpr int kLanes = 4;
+  Mbar ready;
+  ready.init(1);
+  std::atomic<int> abort_cta{1}, looked{0}, at_vote{0}, no{0}, at_sync{0}, at_end{0}, stuck{0};
+  auto meet = [&](std::atomic<int>& count) {
+    count.fetch_add(1);
+    const auto late = clk::now() + std::chrono::seconds(1);
+    while (count.load() < kLanes) {
+      if (clk::now() > late) {
+        stuck.store(1);
+        return;
+      }
+      std::this_thread::yield();
+    }
+  };
+  auto lane = [&](int l) {
+    if (l > 0) while (!looked.load()) std::this_thread::yield();
+    bool ok = ready.wait(0u, [&] { return abort_cta.load() != 0; });  // the phase first, then the flag
+    if (l == 0) {
+      ready.arrive();
+      looked.store(1);
+    }
+    if (uniform) {  // __all_sync
+      if (!ok) no.fetch_add(1);
+      meet(at_vote);
+      ok = no.load() == 0;
+    }
+    if (ok) meet(at_sync);  // the __syncwarp behind the slice's stores
+    meet(at_end);
+  };
+  std::vector<std::thread> th;
+  for (int l = 0; l < kLanes; ++l) th.emplace_back(lane, l);
+  for (auto& x : th) x.join();
+  return stuck.load();
+}

@@ -207,7 +207,7 @@ struct TreeAllReduce {
       for (uint64_t n = 0; n < slices; ++n) {
         const uint32_t g = base + (uint32_t)n;
         const int si = (int)(n % kAhead);
-        if (!gemm::mbar_wait(s_ready + si, (uint32_t)(n / kAhead) & 1u, ab)) break;
+        if (!gemm::agree<false>(gemm::mbar_wait(s_ready + si, (uint32_t)(n / kAhead) & 1u, ab))) break;
         const uint64_t clo = (2 * n + tree) * cv, chi = min(clo + cv, nvec);
         const uint64_t per = (chi - clo + K - 1) / K, lo = min(clo + per * k, chi), hi = min(lo + per, chi);
         // pointers to the slice and 32-bit offsets: 64-bit element numbers cost the registers of the loads

@@ -202,3 +202,13 @@ def test_thread_sanitizer_flags_counters_raised_before_every_data_warp_is_done()
     r = subprocess.run([str(exe), "tree-broken-variant", "4"], capture_output=True, text=True, timeout=300)
     out = r.stdout + r.stderr
     assert "ThreadSanitizer: data race" in out or r.returncode != 0, out[-2000:]
+
+
+def test_lanes_of_a_warp_give_up_a_wait_together():
+    """A wait that one lane gives up and another does not leaves the two at different barriers for good: the time
+    limit of the waits in the chunked tree and in the GEMMs' epilogues holds only because the lanes vote."""
+    from tccl_b200.utils.hostproto import _lib
+
+    lib = _lib()
+    assert lib.hp_selftest_warp_verdict(1) == 0
+    assert lib.hp_selftest_warp_verdict(0) == 1  # every lane for itself: caught
