@@ -93,6 +93,14 @@ class Plan:
 
     def run(self, w, x=None, out=None):
         if self.fresh is not None:  # fresh local output(s) per call
+            if not w.emulated:  # one local rank: no lists (0.3 us of a small call, which pays 0.2 for the lock)
+                shape, strides, dtype, dev = self.fresh
+                o = torch.empty_strided(shape, strides, dtype=dtype, device=dev)
+                with w.lock:
+                    self.structs[0].out = o.data_ptr()
+                    self.go()
+                    w.launches += 1
+                return o
             outs = self.outputs()
             with w.lock:
                 for a, o in zip(self.structs, outs):
