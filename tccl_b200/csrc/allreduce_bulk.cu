@@ -178,10 +178,12 @@ extern "C" int tccl_allreduce_twoshot_bulk(const tccl_comm* comm, const tccl_col
   const int dtype = args->dtype;
   if (l->block != kBulkThreads) return -TCCL_EINVAL;
   const size_t smem = (size_t)(kBulkInStages * world + kBulkOutStages) * bulk_chunk_bytes(world);
-  if (l->n_emu == 0) {
+  const int rc = check_ranks(comm, args, l, [world](const tccl_comm&, const tccl_coll_args& a) {
     for (int p = 0; p < world; ++p)
-      if (((uintptr_t)args->in[p] | (uintptr_t)args->out_peer[p]) & 15) return -TCCL_EALIGN;
-  }
+      if (((uintptr_t)a.in[p] | (uintptr_t)a.out_peer[p]) & 15) return -TCCL_EALIGN;
+    return 0;
+  });
+  if (rc) return rc;
   switch (dtype) {
     case TCCL_BF16: return launch_op<AllReduceTwoShotBulk<__nv_bfloat16>>(comm, args, l, smem);
     case TCCL_F32: return launch_op<AllReduceTwoShotBulk<float>>(comm, args, l, smem);

@@ -196,7 +196,10 @@ static int pipe_entry(const tccl_comm* comm, const tccl_coll_args* args, const t
   const int world = comm->world;
   const int dtype = args->dtype;
   const int pipe_flags = l->meta & ~0xff;
-  if (l->n_emu == 0 && (args->flags & ~0xff) != pipe_flags) return -TCCL_EINVAL;
+  const int rc = check_ranks(comm, args, l, [pipe_flags](const tccl_comm&, const tccl_coll_args& a) {
+    return (a.flags & ~0xff) != pipe_flags ? -TCCL_EINVAL : 0;
+  });
+  if (rc) return rc;
   switch (dtype) {
     case TCCL_BF16: return launch_pipe_world<__nv_bfloat16, kNvls>(comm, args, l, world, pipe_flags);
     case TCCL_F32: return launch_pipe_world<float, kNvls>(comm, args, l, world, pipe_flags);

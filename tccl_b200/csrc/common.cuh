@@ -348,7 +348,21 @@ kernel_real(const __grid_constant__ tccl_comm comm, const __grid_constant__ type
 template <class Args> struct EmuParams {
   tccl_comm comm[TCCL_MAX_WORLD];
   Args args[TCCL_MAX_WORLD];
+  static_assert(TCCL_MAX_WORLD * (sizeof(tccl_comm) + sizeof(Args)) <= 32764, "more than a kernel's parameters may hold");
 };
+
+// A launcher's checks of what it was given, for every rank that the launch drives: the calling one, or all emulated ones.
+// `check(comm, args)` returns 0 or an error code.
+template <class Args, class Check>
+inline int check_ranks(const tccl_comm* comm, const Args* args, const tccl_launch* l, Check check) {
+  if (l->n_emu < 0 || l->n_emu > TCCL_MAX_WORLD) return -TCCL_EINVAL;
+  for (int r = 0; r < (l->n_emu ? l->n_emu : 1); ++r) {
+    if (l->n_emu && comm[r].world != l->n_emu) return -TCCL_EINVAL;
+    const int rc = check(comm[r], args[r]);
+    if (rc) return rc;
+  }
+  return 0;
+}
 template <class Op>
 __global__ void __launch_bounds__(Op::kMaxThreads, Op::kMinBlocks)
 kernel_emu(const __grid_constant__ EmuParams<typename Op::Args> p) {

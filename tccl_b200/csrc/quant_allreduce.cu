@@ -215,10 +215,11 @@ extern "C" uint64_t tccl_allreduce_fp8wire_stage_bytes(uint64_t numel, int world
 // bf16 only; numel % 2048 == 0; l->block == 256; needs tccl_allreduce_fp8wire_stage_bytes() of staging area
 extern "C" int tccl_allreduce_fp8wire(const tccl_comm* comm, const tccl_qar_args* args, const tccl_launch* l) {
   if (l->block != kQThreads) return -TCCL_EINVAL;
-  if (l->n_emu == 0) {
-    if (!args->in || !args->out || args->numel == 0 || args->numel % kQChunk) return -TCCL_ESIZE;
-    if (((uintptr_t)args->in | (uintptr_t)args->out) & 15) return -TCCL_EALIGN;
-    if (QuantAllReduce::bytes_needed(args->numel / kQChunk, comm->world) > comm->stage_bytes) return -TCCL_ESIZE;
-  }
+  const int rc = check_ranks(comm, args, l, [](const tccl_comm& c, const tccl_qar_args& a) {
+    if (!a.in || !a.out || a.numel == 0 || a.numel % kQChunk) return -TCCL_ESIZE;
+    if (((uintptr_t)a.in | (uintptr_t)a.out) & 15) return -TCCL_EALIGN;
+    return QuantAllReduce::bytes_needed(a.numel / kQChunk, c.world) > c.stage_bytes ? -TCCL_ESIZE : 0;
+  });
+  if (rc) return rc;
   return launch_op<QuantAllReduce>(comm, args, l);
 }

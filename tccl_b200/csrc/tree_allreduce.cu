@@ -304,11 +304,13 @@ extern "C" int tccl_allreduce_tree(const tccl_comm* comm, const tccl_tree_args* 
   tccl_launch rounded = *launch;
   rounded.block = launch->block < kTreeCtrl + 32 ? kTreeCtrl + 32 : launch->block / 32 * 32;
   const tccl_launch* l = &rounded;
-  if (l->n_emu == 0) {
-    const int K = args->ctas_per_role;
-    if (K < 1 || K > tree_max_ctas(comm->tree_bytes) || l->grid != 4 * K) return -TCCL_ESIZE;
-    if (args->chunk_vecs < 1 || args->chunk_vecs > (uint64_t)K * (TCCL_TREE_SLICE_BYTES / 16)) return -TCCL_ESIZE;
-  }
+  const int rc = check_ranks(comm, args, l, [l](const tccl_comm& c, const tccl_tree_args& a) {
+    const int K = a.ctas_per_role;
+    if (K < 1 || K > tree_max_ctas(c.tree_bytes) || l->grid != 4 * K) return -TCCL_ESIZE;
+    // a CTA's slice of a chunk stays inside its ring slot
+    return a.chunk_vecs < 1 || a.chunk_vecs > (uint64_t)K * (TCCL_TREE_SLICE_BYTES / 16) ? -TCCL_ESIZE : 0;
+  });
+  if (rc) return rc;
   if (l->meta & TCCL_TREE_PULL_DOWN) {  // on request: children load the sum from their parent
     switch (dtype) {
       case TCCL_BF16: return launch_op<TreeAllReduce<__nv_bfloat16, true>>(comm, args, l);

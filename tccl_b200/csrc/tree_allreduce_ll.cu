@@ -177,13 +177,14 @@ using namespace tccl;
 // args->out may each be null; the other entries of buf are not used.
 extern "C" int tccl_allreduce_tree_ll(const tccl_comm* comm, const tccl_tree_args* args, const tccl_launch* l) {
   const int dtype = args->dtype;
-  if (l->n_emu == 0) {
-    const int K = args->ctas_per_role;
-    const uint64_t esz = args->dtype == TCCL_F32 ? 4 : 2;
+  const int rc = check_ranks(comm, args, l, [l](const tccl_comm& c, const tccl_tree_args& a) {
+    const int K = a.ctas_per_role;
+    const uint64_t esz = a.dtype == TCCL_F32 ? 4 : 2;
     if (K < 1 || K > TCCL_TREE_LL_MAX_CTAS || l->grid != 4 * K) return -TCCL_ESIZE;
-    if (comm->tree_bytes < TCCL_TREE_LL_BYTES) return -TCCL_ESIZE;
-    if (args->numel * esz > 2ull * K * (TCCL_TREE_LL_SLOT_BYTES / 2) || (args->numel * esz) % 16) return -TCCL_ESIZE;
-  }
+    if (c.tree_bytes < TCCL_TREE_LL_BYTES) return -TCCL_ESIZE;
+    return a.numel * esz > 2ull * K * (TCCL_TREE_LL_SLOT_BYTES / 2) || (a.numel * esz) % 16 ? -TCCL_ESIZE : 0;
+  });
+  if (rc) return rc;
   switch (dtype) {
     case TCCL_BF16: return launch_op<TreeAllReduceLL<__nv_bfloat16>>(comm, args, l);
     case TCCL_F32: return launch_op<TreeAllReduceLL<float>>(comm, args, l);
