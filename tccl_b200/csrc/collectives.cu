@@ -119,7 +119,7 @@ struct AllReduceOneShotP2P {
   // one rank: the reduction is a copy; keep it lean so two CTAs fit an SM
   static constexpr int kMaxThreads = 512, kMinBlocks = W == 1 ? 2 : 1;
   static constexpr int kMaxW = W ? W : TCCL_MAX_WORLD;
-  static constexpr int U = W == 1 ? 8 : ((W == 0 || W >= 5) ? 2 : 4);  // vectors per thread per pass
+  static constexpr int U = W == 1 ? 8 : (W >= 5 ? 2 : 4);  // vectors per thread per pass
   static __device__ void run(const tccl_comm& c, const Args& a, int bid, int nb) {
     Entry sync(c, a.flags, bid);
     const int world = WorldOf<W>::get(c);
@@ -299,7 +299,7 @@ struct AllReduceTwoShotP2P {
   using Args = tccl_coll_args;
   static constexpr int kMaxThreads = 512, kMinBlocks = 1;
   static constexpr int kMaxW = W ? W : TCCL_MAX_WORLD;
-  static constexpr int U = (W == 0 || W >= 5) ? 2 : 4;
+  static constexpr int U = W >= 5 ? 2 : 4;
   static __device__ void run(const tccl_comm& c, const Args& a, int bid, int nb) {
     Entry sync(c, a.flags, bid);
     const int world = WorldOf<W>::get(c);
@@ -535,7 +535,7 @@ struct ReduceScatter {
   using Args = tccl_coll_args;
   static constexpr int kMaxThreads = 512, kMinBlocks = 1;
   static constexpr int kMaxW = W ? W : TCCL_MAX_WORLD;
-  static constexpr int U = kNvls ? 8 : ((W == 0 || W >= 5) ? 2 : 4);
+  static constexpr int U = kNvls ? 8 : (W >= 5 ? 2 : 4);
   static __device__ void run(const tccl_comm& c, const Args& a, int bid, int nb) {
     Entry sync(c, a.flags, bid);
     const int world = WorldOf<W>::get(c);
@@ -580,31 +580,47 @@ struct ReduceScatter {
 };
 
 // ------------------------------------------------------------------ dispatchers
-// One instance per world size up to 8: with a run-time count the loads of all 16 possible ranks hold registers and
-// the sums wait behind predicates.  24 MiB of bf16 per rank, one-shot all-reduce / two-shot / reduce-scatter in us,
-// emulated: 3 ranks 54 / 34.5 / 26 run-time, 39 / 31.5 / 22.5 so; 5 ranks 100 / 56 / 32.5 and 79 / 55 / 31; 7 ranks
-// 153 / 75 / 38 and 110 / 75 / 38.
-template <template <typename, int> class Op>
-static int dispatch(const tccl_comm* comm, const tccl_coll_args* args, const tccl_launch* l, int world, int dtype) {
-#define TCCL_W(T)                                                         \
-  switch (world) {                                                        \
-    case 1: return launch_op<Op<T, 1>>(comm, args, l);                    \
-    case 2: return launch_op<Op<T, 2>>(comm, args, l);                    \
-    case 3: return launch_op<Op<T, 3>>(comm, args, l);                    \
-    case 4: return launch_op<Op<T, 4>>(comm, args, l);                    \
-    case 5: return launch_op<Op<T, 5>>(comm, args, l);                    \
-    case 6: return launch_op<Op<T, 6>>(comm, args, l);                    \
-    case 7: return launch_op<Op<T, 7>>(comm, args, l);                    \
-    case 8: return launch_op<Op<T, 8>>(comm, args, l);                    \
-    default: return launch_op<Op<T, 0>>(comm, args, l);                   \
+// Instances: 1, 2, 4 and 8 ranks, and one with a run-time count for the rest.  With a run-time count the loads of all
+// TCCL_MAX_WORLD possible ranks hold registers and the sums wait behind predicates, so the operators that sum over peers
+// with plain loads have an instance for every world size (kEvery).  Emulated, bf16 per rank, run-time -> own instance, us:
+//   one-shot all-reduce  24 MiB at 3 / 5 / 6 / 7 ranks  56.8 / 101 / 129 / 156 -> 43.1 / 82.0 / 102 / 121
+//   two-shot all-reduce   1 MiB                         14.9 / 16.9 / 17.4 / 18.4 -> 14.3 / 16.4 / 16.9 / 18.0; 24 MiB: level
+//   reduce-scatter        1 MiB                         14.5 / 15.2 / 15.4 / 16.4 -> 13.3 / 15.3 / 15.2 / 15.4; 24 MiB
+//                                                       30.9 / 37.9 / 42.0 / 47.1 -> 29.2 / 37.8 / 42.0 / 47.2
+// The others gain nothing from one or lose: push all-reduce and push all-gather are level, the pull all-gather took
+// 69.8 / 175 / 210 / 321 us with the run-time count and 73.8 / 187 / 219 / 337 with instances (24 MiB), and the NVLS
+// forms let the switch do the sum.
+template <template <typename, int> class Op, typename T, bool kEvery>
+static int dispatch_world(const tccl_comm* comm, const tccl_coll_args* args, const tccl_launch* l) {
+  switch (comm->world) {
+    case 1: return launch_op<Op<T, 1>>(comm, args, l);
+    case 2: return launch_op<Op<T, 2>>(comm, args, l);
+    case 4: return launch_op<Op<T, 4>>(comm, args, l);
+    case 8: return launch_op<Op<T, 8>>(comm, args, l);
+    default: break;
   }
-  switch (dtype) {
-    case TCCL_BF16: TCCL_W(__nv_bfloat16)
-    case TCCL_F32: TCCL_W(float)
-    case TCCL_F16: TCCL_W(__half)
+  if constexpr (kEvery) {
+    static_assert(TCCL_MAX_WORLD == 8, "an instance for every world size");
+    switch (comm->world) {
+      case 3: return launch_op<Op<T, 3>>(comm, args, l);
+      case 5: return launch_op<Op<T, 5>>(comm, args, l);
+      case 6: return launch_op<Op<T, 6>>(comm, args, l);
+      case 7: return launch_op<Op<T, 7>>(comm, args, l);
+      default: return -TCCL_EINVAL;
+    }
+  } else {
+    if (comm->world < 1 || comm->world > TCCL_MAX_WORLD) return -TCCL_EINVAL;
+    return launch_op<Op<T, 0>>(comm, args, l);
+  }
+}
+template <template <typename, int> class Op, bool kEvery>
+static int dispatch(const tccl_comm* comm, const tccl_coll_args* args, const tccl_launch* l) {
+  switch (args->dtype) {
+    case TCCL_BF16: return dispatch_world<Op, __nv_bfloat16, kEvery>(comm, args, l);
+    case TCCL_F32: return dispatch_world<Op, float, kEvery>(comm, args, l);
+    case TCCL_F16: return dispatch_world<Op, __half, kEvery>(comm, args, l);
     default: return -TCCL_EDTYPE;
   }
-#undef TCCL_W
 }
 
 template <typename T, int W> using AgPushP2P = AllGatherPush<T, W, false>;
@@ -637,21 +653,21 @@ int tccl_wait_never(const tccl_comm* comm, const tccl_barrier_args* args, const 
   return launch_op<WaitNeverOp>(comm, args, l);
 }
 
-#define TCCL_COLL(name, Op)                                                                   \
+#define TCCL_COLL(name, Op, kEvery)                                                           \
   int name(const tccl_comm* comm, const tccl_coll_args* args, const tccl_launch* l) {         \
-    return dispatch<Op>(comm, args, l, comm->world, args->dtype);                             \
+    return dispatch<Op, kEvery>(comm, args, l);                                               \
   }
-TCCL_COLL(tccl_allreduce_oneshot_p2p, AllReduceOneShotP2P)
-TCCL_COLL(tccl_allreduce_oneshot_nvls, AllReduceOneShotNvls)
-TCCL_COLL(tccl_allreduce_push_p2p, ArPushP2P)
-TCCL_COLL(tccl_allreduce_push_nvls, ArPushNvls)
-TCCL_COLL(tccl_allreduce_twoshot_p2p, AllReduceTwoShotP2P)
-TCCL_COLL(tccl_allreduce_twoshot_nvls, AllReduceTwoShotNvls)
-TCCL_COLL(tccl_allgather_pull_p2p, AllGatherPullP2P)
-TCCL_COLL(tccl_allgather_push_p2p, AgPushP2P)
-TCCL_COLL(tccl_allgather_push_nvls, AgPushNvls)
-TCCL_COLL(tccl_reducescatter_p2p, RsP2P)
-TCCL_COLL(tccl_reducescatter_nvls, RsNvls)
+TCCL_COLL(tccl_allreduce_oneshot_p2p, AllReduceOneShotP2P, true)
+TCCL_COLL(tccl_allreduce_oneshot_nvls, AllReduceOneShotNvls, false)
+TCCL_COLL(tccl_allreduce_push_p2p, ArPushP2P, false)
+TCCL_COLL(tccl_allreduce_push_nvls, ArPushNvls, false)
+TCCL_COLL(tccl_allreduce_twoshot_p2p, AllReduceTwoShotP2P, true)
+TCCL_COLL(tccl_allreduce_twoshot_nvls, AllReduceTwoShotNvls, false)
+TCCL_COLL(tccl_allgather_pull_p2p, AllGatherPullP2P, false)
+TCCL_COLL(tccl_allgather_push_p2p, AgPushP2P, false)
+TCCL_COLL(tccl_allgather_push_nvls, AgPushNvls, false)
+TCCL_COLL(tccl_reducescatter_p2p, RsP2P, true)
+TCCL_COLL(tccl_reducescatter_nvls, RsNvls, false)
 #undef TCCL_COLL
 
 }  // extern "C"

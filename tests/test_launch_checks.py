@@ -86,3 +86,12 @@ def test_emulated_launch_of_another_world_is_refused(name):
     assert _launch(name, _comms(4), make(4), 2, True, **launch) < 0
     assert _launch(name, _comms(2), make(2), -1, True, **launch) < 0
     assert _launch(name, _comms(2), make(2), L.MAX_WORLD + 1, True, **launch) < 0
+
+
+@pytest.mark.parametrize("name", ["tccl_allreduce_oneshot_p2p", "tccl_allreduce_twoshot_p2p", "tccl_reducescatter_p2p",
+                                  "tccl_allgather_pull_p2p", "tccl_allreduce_push_p2p", "tccl_allreduce_oneshot_nvls"])
+def test_world_sizes_without_a_kernel_are_refused(name):
+    for world in (0, -1, L.MAX_WORLD + 1):
+        comms, args = _comms(1), _coll(1)
+        comms[0].world = world
+        assert _launch(name, comms, args, 1, False, grid=8, block=512) < 0
