@@ -231,7 +231,7 @@ def all_reduce(x, out=None, *, inplace: bool = False, algo: str = "auto", world:
         from .tree_allreduce import double_tree_all_reduce
 
         return double_tree_all_reduce(x, out=out, inplace=inplace, world=w)
-    key = ("ar", w.tkey(x), None if out is None else w.tkey(out), inplace, algo, sync_exit)
+    key = ("ar", w.tkey(x), w.okey(out), inplace, algo, sync_exit)
     return _planned(w, key, _plan_all_reduce, x, out, inplace, algo, sync_exit).run(w, x, out)
 
 
@@ -430,7 +430,7 @@ def all_gather(x, out=None, *, algo: str = "auto", world: Optional[WorldBase] = 
     trips), pull otherwise.
     """
     w = get_world(world)
-    key = ("ag", w.tkey(x), None if out is None else w.tkey(out), algo, sync_exit)
+    key = ("ag", w.tkey(x), w.okey(out), algo, sync_exit)
     return _planned(w, key, _plan_all_gather, x, out, algo, sync_exit).run(w, x, out)
 
 
@@ -494,7 +494,7 @@ def reduce_scatter(x, out=None, *, algo: str = "auto", world: Optional[WorldBase
     As in the reference the element count must be a multiple of ``W`` times the
     16-byte vector width (``triton_reduce_scatter.py:102-104``)."""
     w = get_world(world)
-    key = ("rs", w.tkey(x), None if out is None else w.tkey(out), algo, sync_exit)
+    key = ("rs", w.tkey(x), w.okey(out), algo, sync_exit)
     return _planned(w, key, _plan_reduce_scatter, x, out, algo, sync_exit).run(w, x, out)
 
 

@@ -242,3 +242,22 @@ def test_plan_cache_lookups_race_with_evictions():
     cache = Evicting(4)
     cache.insert("a", 1)
     assert cache.lookup("a") == 1 and cache.lookup("a") is None
+
+
+@pytest.mark.parametrize("wrong", ["dtype", "stride"])
+def test_a_destination_of_another_layout_is_refused_on_every_rank(stub, wrong):
+    """A cached launch must not swallow the check of any rank's destination: here rank 1's, at the same address as a good
+    one that was planned before."""
+    w = emulated(stub, 2)
+    x, shares = EmuTensor([_bf16(4096) for _ in range(2)]), [_bf16(4096) for _ in range(2)]
+    bad = shares[1].view(torch.float16) if wrong == "dtype" else shares[1].as_strided((2048,), (2,))
+    cases = [(lambda out: collectives.all_reduce(x, out=out, algo="oneshot_p2p", world=w), 4096),
+             (lambda out: collectives.reduce_scatter(x, out=out, world=w), 2048)]
+    for call, n in cases:
+        call(EmuTensor([s[:n] for s in shares]))
+        with pytest.raises(ValueError):
+            call(EmuTensor([shares[0][:n], bad[:n]]))
+    half = [_bf16(2048) for _ in range(2)]
+    collectives.all_gather(EmuTensor(half), out=EmuTensor(shares), algo="pull", world=w)
+    with pytest.raises(ValueError):
+        collectives.all_gather(EmuTensor(half), out=EmuTensor([shares[0], bad]), algo="pull", world=w)
