@@ -328,7 +328,11 @@ extern "C" int tccl_gemm_reduce_scatter_pair(const tccl_comm* comm, const tccl_g
     if ((args->n % BN2) || (args->m % 128)) return -TCCL_ESIZE;
     const tccl_gemm_args g{args->a, args->bt, args->out, comm->local + TCCL_LOCAL_STATUS, args->m, args->n, args->k,
                            args->lda, args->ldb, args->ldo, 0};
-    return launch_gemm_pair(&g, args->trace ? l->grid : 0, s, comm->timeout_ns, reinterpret_cast<uint64_t*>(args->trace));
+    // a grid short of the whole GPU is the caller's limit on CTAs (and a traced launch has a row of words per CTA):
+    // only without one is the kernel that suits the shape free to choose its own
+    const bool limited = l->grid < (tccl_num_sms() & ~1);
+    return launch_gemm_pair(&g, args->trace || limited ? l->grid : 0, s, comm->timeout_ns,
+                            reinterpret_cast<uint64_t*>(args->trace));
   }
   static bool attr_set = false;
   if (!attr_set) {

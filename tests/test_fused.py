@@ -220,3 +220,36 @@ def test_one_rank_rows_short_of_a_pair_tile(emu_worlds, M, swiglu):
         w.check()
         err = (full[:M].float() - ref).abs()
         assert bool((err <= ref.abs() * 2 ** -8 + sums).all()) and bool((full[M:] == 77.0).all())
+
+
+def test_one_rank_reduce_scatter_keeps_to_its_grid():
+    """A limit on CTAs holds at one rank too: a pair of SMs takes many times as long as all of them (the product is also
+    one that the kernel for few tiles would take)."""
+    import ctypes as C
+
+    from tccl_b200.utils import lib as L
+
+    M, N, K = 512, 2048, 4096
+    a, bt, out = _rand((M, K), 1), _rand((N, K), 2, 0.02), torch.empty(M, N, dtype=torch.bfloat16, device="cuda")
+    local = torch.zeros(L.K["TCCL_LOCAL_WORDS"], dtype=torch.int32, device="cuda")
+    comm = L.Comm()
+    comm.world, comm.rank, comm.local, comm.timeout_ns = 1, 0, local.data_ptr(), 5_000_000_000
+    g = L.GemmRsArgs(a.data_ptr(), bt.data_ptr(), out.data_ptr(), M, N, K, K, K, N, 0)
+    stream = torch.cuda.current_stream().cuda_stream
+    ref = a.float() @ bt.float().t()
+
+    def run(grid):
+        times = []
+        for _ in range(5):
+            t0, t1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            t0.record()
+            l = L.Launch(grid, 256, 0, 0, stream)
+            assert L.lib().tccl_gemm_reduce_scatter_pair(C.byref(comm), C.byref(g), C.c_uint64(0), C.byref(l)) == 0
+            t1.record()
+            t1.synchronize()
+            times.append(t0.elapsed_time(t1))
+        err = (out.float() - ref).abs()
+        assert bool((err <= ref.abs() * 2 ** -8 + 1e-3 * (K ** 0.5) * 0.02).all())
+        return min(times)
+
+    assert run(2) > 4 * run(L.lib().tccl_num_sms() & ~1)
