@@ -68,8 +68,8 @@ __device__ __forceinline__ void skinny_reduce(const SkinnyArgs& p, uint32_t part
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       const int i = i0 + u * kThreads, tok = i / kVpt * S + s;
-      // only what is stored below is loaded: a load that nothing waits for could outlive the CTA it reads from
-      if (i < kTotal && tok0 + tok < p.M && rt * kCols + i % kVpt * 4 < p.N) {
+      // from another CTA only what is stored below is loaded: a load that nothing waits for could outlive that CTA
+      if (i < kTotal && tok0 + tok < p.M && (S == 1 || rt * kCols + i % kVpt * 4 < p.N)) {
         const uint32_t off = part0 + (uint32_t)(tok * kSkinnyRows + i % kVpt * 4) * 4;
 #pragma unroll
         for (int q = 0; q < S; ++q) {
@@ -259,11 +259,13 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
 #undef TCCL_SKINNY_REDUCE
   // Nobody leaves while another CTA of the cluster may still read its partial, or while the leader's commits are still on
   // their way to this CTA's barriers: each lane looks at the last phase of one stage's (all landed long ago, unless a wait
-  // failed; a thread that waited for one stage after the other where the loads end cost 1.5 us, this 0.2).
+  // failed; a thread that waited for one stage after the other where the loads end cost 1.5 us).
+  __syncthreads();
+  if (cl > 1) cluster_arrive_relaxed();
   if (CG == 2 && !leader && warp == 0 && lane < NS && lane < kb1 - kb0)
     drain_ring(empty + lane, 1, (uint32_t)((kb1 - kb0 - 1 - lane) / NS + 1), !*ab.flag, p.timeout_ns);
-  __syncthreads();
-  if (cl > 1) cluster_sync_relaxed();
+  __syncwarp();
+  if (cl > 1) cluster_wait();
   if (warp == 2) {
     tc_fence_after();
     if (CG == 2) tmem_dealloc2(tmem, Cfg::kTmem);

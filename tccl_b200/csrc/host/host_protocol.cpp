@@ -1200,12 +1200,12 @@ extern "C" int hp_selftest_tree_ll(int world, int numel, int calls, int depth) {
 // ---------------------------------------------------------------------------
 // Model of how a CTA pair ends (gemm_tcgen05_2cta.cuh, gemm_skinny.cu).  The epilogue of the second CTA arrives on the
 // leader's tmem_empty barriers and the leader's MMA thread commits to the second CTA's empty barriers; such remote
-// arrivals travel through an INTERCONNECT thread that delivers them later than they are issued.  Both CTAs then meet at
-// a cluster barrier that orders only their own threads, and what a CTA leaves behind is taken over by the next one
-// (`rounds` pairs run one after the other on the same two shared memories).  The accumulators and stages used last are
-// reused by nobody, so nothing in the mainloop waits for the arrivals that free them: `drain` = 1 (the kernels) waits for
-// their last phases before the cluster barrier; `drain` = 0 is the mistake, kept so that the sanitizer can be seen to
-// catch it: a late arrival hits the shared memory of the next CTA.
+// arrivals travel through an INTERCONNECT thread that delivers them later than they are issued.  Both CTAs meet at a
+// split cluster barrier whose arrival is relaxed, and what a CTA leaves behind is taken over by the next one (`rounds`
+// pairs run one after the other on the same two shared memories).  The accumulators and stages used last are reused by
+// nobody, so nothing in the mainloop waits for the arrivals that free them: `drain` = 1 (the kernels) waits for their
+// last phases between the barrier's halves; `drain` = 0 is the mistake, kept so that the sanitizer can be seen to catch
+// it: a late arrival hits the shared memory of the next CTA.
 namespace {
 struct PairSmem {
   Mbar full[2], empty[2], tmem_full[2], tmem_empty[2];
@@ -1251,29 +1251,29 @@ extern "C" int hp_selftest_pair_exit(int tiles, int rounds, int drain) {
   PairSmem sm[2];
   Interconnect net((size_t)rounds * tiles * 4 + 4);
   std::thread wire([&] { net.run(); });
-  KernelBoundary edge;
+  KernelBoundary start, own_cta[2];
+  std::atomic<int> at_end{0};  // relaxed arrivals at the pair's last barrier
   // a stray arrival leaves a barrier out of step: nobody waits on after one (or after ten seconds)
   const auto give_up = clk::now() + std::chrono::seconds(10);
-  auto await = [&](const Mbar& b, uint32_t parity) {
-    while ((b.phase.load(std::memory_order_acquire) & 1u) == parity && !net.strays.load(std::memory_order_relaxed)) {
-      if (clk::now() > give_up) net.strays.fetch_add(1);
-      std::this_thread::yield();
-    }
+  auto lost = [&] {
+    if (clk::now() > give_up) net.strays.fetch_add(1);
+    return net.strays.load(std::memory_order_relaxed) != 0;
   };
+  auto await = [&](const Mbar& b, uint32_t parity) { b.wait(parity, lost); };
   auto cta = [&](int c, int role) {
-    int sense = 0;
+    int sense = 0, cta_sense = 0;
     for (int round = 1; round <= rounds && !net.strays.load(); ++round) {
-      if (c == 0 && role == 0)
-        for (PairSmem& s : sm) {  // the next pair's CTAs set up the shared memory they were given
-          s.owner = (uint32_t)round;
-          for (int i = 0; i < 2; ++i) {
-            s.full[i].init(2);
-            s.empty[i].init(1);
-            s.tmem_full[i].init(1);
-            s.tmem_empty[i].init(2);
-          }
+      if (role == 0) {  // the next CTA sets up the shared memory it was given
+        PairSmem& s = sm[c];
+        s.owner = (uint32_t)round;
+        for (int i = 0; i < 2; ++i) {
+          s.full[i].init(2);
+          s.empty[i].init(1);
+          s.tmem_full[i].init(1);
+          s.tmem_empty[i].init(2);
         }
-      edge.arrive_and_wait(6, sense, &net.strays);  // producer, MMA (or idle) and epilogue threads of both CTAs
+      }
+      start.arrive_and_wait(6, sense, &net.strays);  // producer, MMA (or idle) and epilogue threads of both CTAs
       const uint32_t own = (uint32_t)round;
       auto parity = [](int use) { return ((uint32_t)use & 1u) ^ 1u; };  // of a ring of two, before its use / 2-th filling
       if (role == 0) {  // producer: one stage per tile; the bytes of both CTAs are counted on the leader's barrier
@@ -1282,7 +1282,6 @@ extern "C" int hp_selftest_pair_exit(int tiles, int rounds, int drain) {
           if (c == 0) sm[0].full[t & 1].arrive();
           else net.arrive(&sm[0], &sm[0].full[t & 1], own);
         }
-        for (int t = tiles; drain && t < tiles + 2; ++t) await(sm[c].empty[t & 1], parity(t >> 1));
       } else if (role == 1 && c == 0) {  // the leader's MMA thread
         for (int t = 0; t < tiles; ++t) {
           await(sm[0].tmem_empty[t & 1], parity(t >> 1));
@@ -1292,7 +1291,6 @@ extern "C" int hp_selftest_pair_exit(int tiles, int rounds, int drain) {
           sm[0].tmem_full[t & 1].arrive();
           net.arrive(&sm[1], &sm[1].tmem_full[t & 1], own);
         }
-        for (int t = tiles; drain && t < tiles + 2; ++t) await(sm[0].tmem_empty[t & 1], parity(t >> 1));
       } else if (role == 2) {  // epilogue
         for (int t = 0; t < tiles; ++t) {
           await(sm[c].tmem_full[t & 1], (uint32_t)(t >> 1) & 1u);
@@ -1300,7 +1298,14 @@ extern "C" int hp_selftest_pair_exit(int tiles, int rounds, int drain) {
           else net.arrive(&sm[0], &sm[0].tmem_empty[t & 1], own);
         }
       }
-      edge.arrive_and_wait(6, sense, &net.strays);  // both CTAs leave together
+      own_cta[c].arrive_and_wait(3, cta_sense, &net.strays);  // __syncthreads
+      at_end.fetch_add(1, std::memory_order_relaxed);
+      for (int t = tiles; drain && t < tiles + 2; ++t) {
+        if (role == 0) await(sm[c].empty[t & 1], parity(t >> 1));
+        if (role == 1 && c == 0) await(sm[0].tmem_empty[t & 1], parity(t >> 1));
+      }
+      while (at_end.load(std::memory_order_acquire) < 6 * round && !lost()) std::this_thread::yield();
+      own_cta[c].arrive_and_wait(3, cta_sense, &net.strays);  // the CTA is gone, its SM is free
     }
   };
   std::vector<std::thread> th;
