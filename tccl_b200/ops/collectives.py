@@ -87,21 +87,17 @@ class Plan:
         # half the host time of empty (1.1 against 2.1 us).
         self.fresh = None if fresh is None else (fresh[0], _dense_strides(fresh[0]), fresh[1], fresh[2])
 
-    def outputs(self):
-        shape, strides, dtype, dev = self.fresh
-        return [torch.empty_strided(shape, strides, dtype=dtype, device=dev) for _ in self.structs]
-
     def run(self, w, x=None, out=None):
         if self.fresh is not None:  # fresh local output(s) per call
+            shape, strides, dtype, dev = self.fresh
             if not w.emulated:  # one local rank: no lists (0.3 us of a small call, which pays 0.2 for the lock)
-                shape, strides, dtype, dev = self.fresh
                 o = torch.empty_strided(shape, strides, dtype=dtype, device=dev)
                 with w.lock:
                     self.structs[0].out = o.data_ptr()
                     self.go()
                     w.launches += 1
                 return o
-            outs = self.outputs()
+            outs = [torch.empty_strided(shape, strides, dtype=dtype, device=dev) for _ in self.structs]
             with w.lock:
                 for a, o in zip(self.structs, outs):
                     a.out = o.data_ptr()
@@ -231,7 +227,7 @@ def all_reduce(x, out=None, *, inplace: bool = False, algo: str = "auto", world:
         from .tree_allreduce import double_tree_all_reduce
 
         return double_tree_all_reduce(x, out=out, inplace=inplace, world=w)
-    key = ("ar", w.tkey(x), w.okey(out), inplace, algo, sync_exit)
+    key = ("ar", w.tkey(x), None if out is None else w.okey(out), inplace, algo, sync_exit)
     return _planned(w, key, _plan_all_reduce, x, out, inplace, algo, sync_exit).run(w, x, out)
 
 
@@ -430,7 +426,7 @@ def all_gather(x, out=None, *, algo: str = "auto", world: Optional[WorldBase] = 
     trips), pull otherwise.
     """
     w = get_world(world)
-    key = ("ag", w.tkey(x), w.okey(out), algo, sync_exit)
+    key = ("ag", w.tkey(x), None if out is None else w.okey(out), algo, sync_exit)
     return _planned(w, key, _plan_all_gather, x, out, algo, sync_exit).run(w, x, out)
 
 
@@ -494,7 +490,7 @@ def reduce_scatter(x, out=None, *, algo: str = "auto", world: Optional[WorldBase
     As in the reference the element count must be a multiple of ``W`` times the
     16-byte vector width (``triton_reduce_scatter.py:102-104``)."""
     w = get_world(world)
-    key = ("rs", w.tkey(x), w.okey(out), algo, sync_exit)
+    key = ("rs", w.tkey(x), None if out is None else w.okey(out), algo, sync_exit)
     return _planned(w, key, _plan_reduce_scatter, x, out, algo, sync_exit).run(w, x, out)
 
 

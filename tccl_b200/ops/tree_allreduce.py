@@ -68,7 +68,7 @@ def _tree_grid(w: WorldBase, nbytes: int):
 
 def double_tree_all_reduce(tensor, out=None, *, inplace: bool = False, world: Optional[WorldBase] = None):
     w = get_world(world)
-    key = ("tree", w.tkey(tensor), w.okey(out), inplace)
+    key = ("tree", w.tkey(tensor), None if out is None else w.okey(out), inplace)
     return _planned(w, key, _plan, tensor, out, inplace).run(w, tensor, out)
 
 

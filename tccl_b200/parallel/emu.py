@@ -141,8 +141,8 @@ class EmuWorld(WorldBase):
         x0 = x.parts[0]
         return (tuple([p.data_ptr() for p in x.parts]), x0.shape, x0.stride(), x0.dtype)
 
-    def okey(self, out) -> Optional[tuple]:
-        return None if out is None else tuple([(p.data_ptr(), p.shape, p.stride(), p.dtype) for p in out.parts])
+    def okey(self, out: EmuTensor) -> tuple:
+        return tuple([(p.data_ptr(), p.numel(), p.dtype, p.is_contiguous()) for p in out.parts])
 
     def stage_ptrs(self) -> List[int]:
         return [s.data_ptr() for s in self.stages]

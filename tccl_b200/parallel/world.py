@@ -120,9 +120,9 @@ class WorldBase:
         must not hit that tensor's plan."""
         return (x.data_ptr(), x.shape, x.stride(), x.dtype)
 
-    def okey(self, out) -> Optional[tuple]:
-        """:meth:`tkey` of the caller's ``out`` or None: plans check every local rank's part of it."""
-        return None if out is None else self.tkey(out)
+    def okey(self, out) -> tuple:
+        """:meth:`tkey` of the caller's ``out``: what plans check in it, of every local rank's part."""
+        return self.tkey(out)
 
     def wrap(self, per_rank: List[torch.Tensor]):
         """Turn the local ranks' tensors into what this world hands back to the user."""

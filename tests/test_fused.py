@@ -253,3 +253,36 @@ def test_one_rank_reduce_scatter_keeps_to_its_grid():
         return min(times)
 
     assert run(2) > 4 * run(L.lib().tccl_num_sms() & ~1)
+
+
+@pytest.mark.parametrize("W", [1, 2, 4])
+def test_callers_buffers_at_new_addresses(emu_worlds, W):
+    """Symmetric buffers of the caller's, others on every call of one shape: each call fills its own and leaves those of
+    earlier calls alone."""
+    import tccl_b200 as tccl
+    from tccl_b200.utils.numerics import allreduce_rmsnorm_check
+
+    w = emu_worlds(W)
+    M, N, K, H = 512 * W, 256, 128, 1024
+    bt = [_rand((N, K), 7100 + r, 0.05) for r in range(W)]
+    wn = [_rand((H,), 7200)] * W
+    kept = []
+    for call in range(3):
+        shards = [_rand((M // W, K), 7300 + 10 * call + r) for r in range(W)]
+        full = w.empty((M, K), torch.bfloat16)
+        outs, got = tccl.all_gather_gemm(shards, bt, a_full=full, world=w)
+        assert got is full
+        x, y, h = (w.empty((8 * W, H), torch.bfloat16) for _ in range(3))
+        for r in range(W):
+            x.parts[r].copy_(_rand((8 * W, H), 7400 + 10 * call + r))
+        assert tccl.all_reduce_bias_residual_rmsnorm(x, wn, out=y, residual_out=h, world=w) == (y, h)
+        kept.append((torch.cat(shards), full, outs, x, y, h))
+    torch.cuda.synchronize()
+    w.check()
+    for a_all, full, outs, x, y, h in kept:
+        s = sum(p.float() for p in x.parts)
+        for r in range(W):
+            assert torch.equal(full[r], a_all)
+            prod = a_all.float() @ bt[r].float().t()
+            assert bool(((outs[r].float() - prod).abs() <= prod.abs() * 2 ** -8 + 1e-3 * (K ** 0.5) * 0.05).all())
+            assert allreduce_rmsnorm_check(y[r], h[r], s, None, None, wn[0], 1e-5, W, False)[0]
