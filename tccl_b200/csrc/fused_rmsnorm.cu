@@ -57,7 +57,8 @@ struct AllReduceRmsNorm {
     const int warp = t >> 5, lane = t & 31, nwarps = nt >> 5;
     // Everything that does not wait for a result is loaded ahead of it: weight and bias once, before the barrier, and a
     // row's residual before its partial sums.  Loaded where they are used, the three took a round trip each per row
-    // (one rank, bf16, with residual: 2048 x 4096 23.1 -> 19.7 us, 2048 x 1024 12.4 -> 10.4).
+    // (one rank, bf16, with residual: 2048 x 4096 23.1 -> 19.7 us, 2048 x 1024 12.4 -> 10.4).  Above hidden 8192 they cost
+    // 40 - 48 bytes of spills and pay all the same: 2048 x 16384 122.9 -> 84.0 us with the one-rank barrier gone as well.
     Vec16 wr[kMaxVec], br[kMaxVec];
 #pragma unroll
     for (int j = 0; j < kMaxVec; ++j) {

@@ -77,7 +77,7 @@ __host__ __device__ __forceinline__ int tree_max_ctas(uint64_t tree_bytes) {
 template <typename T, bool kPullDown>
 struct TreeAllReduce {
   using Args = tccl_tree_args;
-  static constexpr int kMaxThreads = 512, kMinBlocks = 1;  // (576 would leave 96 registers a thread: spills)
+  static constexpr int kMaxThreads = 512, kMinBlocks = 1;  // 128 registers a thread: up to 16 bytes of spills (576: 96)
   static constexpr int kAhead = 4;  // slices between polling and posting
   static constexpr int U = 4;  // vectors in flight per thread and source
 

@@ -156,7 +156,8 @@ def build_host_tsan(verbose: bool = False) -> Path:
 
 def ptxas_table() -> str:
     """Registers, spills and static shared memory of every kernel, as ptxas reports them
-    (``-Xptxas -v``), one markdown row per kernel template: the instance with the most registers."""
+    (``-Xptxas -v``), one markdown row per kernel template: the most registers and the worst spills of any
+    of its instances (not always the same one), and how many instances spill."""
     import re
     import tempfile
 
@@ -188,16 +189,14 @@ def ptxas_table() -> str:
                     fam = fam.replace("(__nv_bfloat16)", "").replace("tccl::", "")
                     fam = re.sub(r"__nv_bfloat16|__half|float", "T", fam)
                     regs, smem = int(m.group(1)), int(m.group(4) or 0)
-                    cur = rows.get((src.name, fam))
-                    if cur is None or regs > cur[0]:
-                        rows[(src.name, fam)] = (regs, spill, smem, (cur[3] if cur else 0) + 1)
-                    else:
-                        rows[(src.name, fam)] = (cur[0], cur[1], cur[2], cur[3] + 1)
-                    entry = None
-    out = ["| source | kernel (template arguments folded) | instances | max registers | stack / spill st / spill ld (B) | static smem (B) |",
+                    cur = rows.get((src.name, fam), (0, (0, 0, 0), 0, 0, 0))
+                    rows[(src.name, fam)] = (max(regs, cur[0]), max(spill, cur[1], key=lambda v: v[1:]), max(smem, cur[2]),
+                                             cur[3] + 1, cur[4] + (spill[1] > 0 or spill[2] > 0))
+                    entry, spill = None, (0, 0, 0)
+    out = ["| source | kernel (template arguments folded) | instances (that spill) | max registers | worst stack / spill st / spill ld (B) | static smem (B) |",
            "|---|---|---|---|---|---|"]
-    for (src, fam), (regs, spill, smem, cnt) in sorted(rows.items()):
-        out.append(f"| `{src}` | `{fam}` | {cnt} | {regs} | {spill[0]} / {spill[1]} / {spill[2]} | {smem} |")
+    for (src, fam), (regs, spill, smem, cnt, spills) in sorted(rows.items()):
+        out.append(f"| `{src}` | `{fam}` | {cnt}{f' ({spills})' if spills else ''} | {regs} | {spill[0]} / {spill[1]} / {spill[2]} | {smem} |")
     return "\n".join(out)
 
 
