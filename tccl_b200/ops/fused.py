@@ -50,9 +50,10 @@ class FusedPlan:
     """A validated launch of a fused kernel for one layout of its operands: argument structs, one per local rank in
     one array, and the launcher.  Every call writes the addresses of its own operands into the structs, so tensors
     at new addresses cost what known ones do: 11 us of host time for the RMSNorm operator.  (Keyed on addresses it
-    was 9 on known ones and 30 on new ones, more than the 18 without any plan.)  ``fresh`` = (shape, strides) of the output that a call allocates when the caller gives none;
-    ``views``: buffers of the communicator's own that a call hands out.  The structs are shared by all calls of the plan:
-    they are written and launched under one hold of the communicator's lock."""
+    was 9 on known ones and 30 on new ones, more than the 18 without any plan.)  ``fresh`` = (shape, strides) of the
+    output that a call allocates when the caller gives none; ``views``: buffers of the communicator's own that a call
+    hands out.  The structs are shared by all calls of the plan: they are written and launched under one hold of the
+    communicator's lock."""
 
     __slots__ = ("arr", "l", "call", "name", "fresh", "user", "views")
 

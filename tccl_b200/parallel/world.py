@@ -132,9 +132,10 @@ class WorldBase:
                 dtype_code: int = 0):
         """Bind one kernel launch to its arguments; returns a zero-argument callable
         that enqueues it on the current stream, to be called with ``lock`` held; the caller counts it in
-        ``launches``.  It keeps no reference to the communicator, which keeps the cached launches.    The caller may patch a
-        field (an output pointer) of ``args_by_rank``'s structs before a call, under the same hold of the
-        lock; a world may replace the dict's values by structs of its own, so they are looked up there again."""
+        ``launches``.  It keeps no reference to the communicator, which keeps the cached launches.  The
+        caller may patch a field (an output pointer) of ``args_by_rank``'s structs before a call, under the
+        same hold of the lock; a world may replace the dict's values by structs of its own, so they are
+        looked up there again."""
         raise NotImplementedError
 
     def comm_ref(self):
